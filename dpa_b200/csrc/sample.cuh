@@ -76,10 +76,11 @@ struct Weights {
   float2 w21;
 };
 
-// fmod(a, h) from the floor s of the rounded quotient a / h.
+// fmod(a, h) from the floor s of the rounded quotient a / h. (A negative a is
+// inside only where a / h underflows to -0; fmod(a, h) is then a itself.)
 __device__ __forceinline__ float remainder_general(float a, float s, float h) {
   float r = fmaf(-s, h, a);
-  if (r < 0.0f) r = __fadd_rn(r, h);
+  if (r < 0.0f && a > 0.0f) r = __fadd_rn(r, h);
   if (r == 0.0f) r = copysignf(0.0f, a);
   return r;
 }
