@@ -33,9 +33,10 @@ struct CurveCounter {
   }
 };
 
-template <int kIntegrator, bool kUnsteady, int kPPT>
+template <int kIntegrator, bool kRecord, bool kUnsteady, int kPPT>
 constexpr int advect_min_blocks() {
   return kPPT == 2                                       ? kAdvectPpt2MinBlocks
+         : kRecord && !kUnsteady                         ? kAdvectRecordMinBlocks
          : kUnsteady                                     ? kAdvectUnsteadyMinBlocks
          : kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4_TRUE ? kAdvectTrueRk4MinBlocks
                                                          : kAdvectMinBlocks;
@@ -60,7 +61,7 @@ constexpr int advect_min_blocks() {
 // particle per lane the branch-free steady Euler and RK4 steppers step a
 // parked slot and discard the result; otherwise an empty slot takes no steps.
 template <int kIntegrator, int kStorage, int kLocate, bool kRecord, bool kUnsteady, int kPPT>
-__global__ void __launch_bounds__(kAdvectBlock, advect_min_blocks<kIntegrator, kUnsteady, kPPT>())
+__global__ void __launch_bounds__(kAdvectBlock, advect_min_blocks<kIntegrator, kRecord, kUnsteady, kPPT>())
 advect_kernel(const FieldView f, const AdvectArgs a) {
   using Sampler = std::conditional_t<kUnsteady, TimeSampler<kStorage, kLocate>,
                                      CellSampler<kStorage, kLocate>>;

@@ -640,13 +640,16 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     }
     v.stride0 = uint32_t(shape[1] * shape[2]);
     v.stride1 = uint32_t(shape[2]);
-    v.node_bias = 0x4B000000u * (v.stride0 + v.stride1 + 1u);
+    v.unit[0] = v.unit[1] = 1.0f;
     v.storage = storage;
     v.locate = dpa::kLocatePow2;
     if (!pow2 && ctx->ieee_division) {
       v.locate = dpa::kLocateDivide;
     } else if (!pow2) {
+      // The range that locate()'s single test of the dividends rests on.
       bool exact = true;
+      for (int i = 0; i < 3; ++i)
+        exact = exact && spacing[i] >= std::ldexp(1.0f, -40) && spacing[i] <= std::ldexp(1.0f, 40);
       for (int i = 0; i < 3 && exact; ++i) {
         const int st = reciprocal_divides_exactly(ctx, spacing[i], &exact);
         if (st != DPA_OK) {

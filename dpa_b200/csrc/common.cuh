@@ -29,7 +29,8 @@ constexpr float kZeroPrecision = 1e-5f;
 //   kLocateReciprocal  a / h as one product and one FMA with the reciprocal
 //                      split in two floats (divide_by_reciprocal), used only
 //                      for divisors for which it was checked at field creation
-//                      to equal __fdiv_rn for every float a;
+//                      to equal __fdiv_rn for every float a (and for spacings
+//                      in [2^-40, 2^40]);
 //   kLocatePow2        power-of-two spacing: one FMA of the exact p / h and
 //                      offset / h, and fmod(p - offset, h) / h = q - floor(q).
 enum LocateMode : int { kLocateDivide = 0, kLocateReciprocal = 1, kLocatePow2 = 2 };
@@ -50,9 +51,7 @@ struct FieldView {
   float scaled_offset[3];  // offset / spacing, exact; used by kLocatePow2 only
   float upper[3];          // n - 1: inside iff 0 <= (p - offset) / h < n - 1
   uint32_t cells[3];       // n - 1, the cells per axis
-  // (2^23 as float bits) * (stride0 + stride1 + 1), modulo 2^32: what the
-  // cell index subtracts when it is formed from biased floors (sample.cuh).
-  uint32_t node_bias;
+  float unit[2];           // {1, 1}: a multiplier the compiler cannot see (sample.cuh)
   int32_t storage;         // dpa_storage
   // LocateMode of the spatial axes. kLocatePow2 needs every spacing a power
   // of two in [2^-20, 2^20] and every offset zero or at least 2^-100 in
@@ -88,25 +87,6 @@ template <int kLocate>
 __device__ __forceinline__ float divide_spacing(float a, float h, float y, float yl) {
   if constexpr (kLocate == kLocateDivide) return __fdiv_rn(a, h);
   else return divide_by_reciprocal(a, h, y, yl);
-}
-
-// Three divisions by known divisors (a_i / h_i, reciprocal pairs y_i, yl_i):
-// one range test for all three dividends instead of one each. Inside the
-// range every quotient is the reciprocal form's, as divide_by_reciprocal
-// gives; otherwise each takes divide_by_reciprocal's own test. (fminf and
-// fmaxf pass over NaN, but a NaN dividend gives NaN on either path.)
-__device__ __forceinline__ void divide3_by_reciprocal(const float a[3], const float h[3],
-                                                      const float y[3], const float yl[3],
-                                                      float q[3]) {
-  const float lo = fminf(fminf(fabsf(a[0]), fabsf(a[1])), fabsf(a[2]));
-  const float hi = fmaxf(fmaxf(fabsf(a[0]), fabsf(a[1])), fabsf(a[2]));
-  if (lo >= 0x1p-64f && hi <= 0x1p64f) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) q[i] = __fmaf_rn(a[i], y[i], __fmul_rn(a[i], yl[i]));
-  } else {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) q[i] = divide_by_reciprocal(a[i], h[i], y[i], yl[i]);
-  }
 }
 
 // Integrator id of the kernel instantiation shared by the reference's other

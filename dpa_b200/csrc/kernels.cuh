@@ -19,6 +19,11 @@ constexpr int kAdvectMinBlocks = DPA_ADVECT_MIN_BLOCKS;
 #define DPA_ADVECT_UNSTEADY_MIN_BLOCKS 2
 #endif
 constexpr int kAdvectUnsteadyMinBlocks = DPA_ADVECT_UNSTEADY_MIN_BLOCKS;
+// Recording keeps the curve's end and counters as well: up to 80 registers
+// instead of spilling in the step at 64. A launch's length is its longest
+// particle's chain of steps, and few pieces of a round have particles enough
+// for a fourth block.
+constexpr int kAdvectRecordMinBlocks = 3;
 // Four-sample RK4 keeps three more stage derivatives alive: up to 80
 // registers (3 blocks per SM) instead of spilling at 64.
 #ifndef DPA_ADVECT_TRUE_RK4_MIN_BLOCKS

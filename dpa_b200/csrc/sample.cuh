@@ -11,10 +11,6 @@
 
 #include "common.cuh"
 
-// F32 trilinear products as packed FMUL2 pairs (1) or scalar FMULs (0).
-#ifndef DPA_F32_PACKED_LERP
-#define DPA_F32_PACKED_LERP 0
-#endif
 
 namespace dpa {
 
@@ -43,24 +39,26 @@ __device__ __forceinline__ void load_node(const void* nodes, int64_t index, floa
 }
 
 // Two FP32 lanes. Products use sm_100's packed multiply (FMUL2), whose
-// lanes round exactly as __fmul_rn does. Sums that may take such a product
-// as an operand stay scalar (__fadd_rn): the compiler fuses a packed multiply
+// lanes round exactly as __fmul_rn does. The compiler fuses a packed multiply
 // feeding a packed add into one packed FMA even when both carry explicit
 // round-to-nearest, and the fused result differs from the reference's
-// separately rounded product and sum. sum2 is the packed add for operands
-// that are never products.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+// separately rounded product and sum. A sum that may take such a product as an
+// operand is therefore a * unit + b in one packed FMA whose multiplier, 1.0,
+// comes with the launch (FieldView::unit): the product by 1 is exact, so the
+// FMA rounds a + b once, and a multiplier unknown when compiling leaves nothing
+// to fuse.
+__device__ __forceinline__ float2 add2(float2 a, float2 b, float2 unit) {
+  return __ffma2_rn(a, unit, b);
 }
-__device__ __forceinline__ float2 sum2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-// Two scalar products, for lerps whose operands would need extra register
-// moves to form the pairs a packed multiply reads.
-__device__ __forceinline__ float2 mul2_scalar(float2 a, float2 b) {
-  return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
-}
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
+// t * a + u * b, every operation rounded on its own.
+__device__ __forceinline__ float2 blend2(float2 a, float2 b, float2 t, float2 u, float2 unit) {
+  return add2(mul2(t, a), mul2(u, b), unit);
+}
+__device__ __forceinline__ float blend(float a, float b, float t, float u) {
+  return __fadd_rn(__fmul_rn(t, a), __fmul_rn(u, b));
+}
 
 // A particle position is held as p0 and the pair p21 = (p2, p1): the
 // derivative of (p2, p1) is (v0, v1), the first two components of a sample,
@@ -85,6 +83,11 @@ __device__ __forceinline__ float remainder_general(float a, float s, float h) {
   return r;
 }
 
+// Subscripts of a cell's first node.
+struct Cell {
+  uint32_t i0, i1, i2;
+};
+
 // Where a position falls in the grid, per axis: the rounded quotient
 // q = (p - offset) / h, its floor s (the cell subscript) and the weight
 // w = fmod(p - offset, h) / h, all as the reference rounds them. The position
@@ -92,8 +95,8 @@ __device__ __forceinline__ float remainder_general(float a, float s, float h) {
 // for any float q (NaN included) is 0 <= q < n - 1.
 //
 // kLocatePow2: q is one FMA of the exact p / h and offset / h, and
-// fmod(a, h) / h = q - s, whose difference is representable; the sign of a
-// zero weight follows q as fmod's follows a.
+// fmod(a, h) / h = q - s, whose difference is representable; a zero weight
+// takes q's sign as fmod's takes a's (q - s is -0 - (+0) = -0 for q = -0).
 //
 // Other spacings: the rounded quotient is either the true integer quotient N
 // or N + 1 (only when a / h lies within half an ulp below N + 1, so that
@@ -101,120 +104,125 @@ __device__ __forceinline__ float remainder_general(float a, float s, float h) {
 // one FMA gives it exactly; adding h back in the N + 1 case is exact too.
 // Both divisions are IEEE division (kLocateDivide) or by the verified
 // reciprocal pair (kLocateReciprocal), which gives the same bits.
-template <int kLocate>
-__device__ __forceinline__ float weight_general(float a, float s, float h, float y, float yl) {
-  return divide_spacing<kLocate>(remainder_general(a, s, h), h, y, yl);
+//
+// kLocateReciprocal's fields have spacings in [2^-40, 2^40]. One test, every
+// a >= 2^-64, then covers both divisions: a quotient beyond divide_by_
+// reciprocal's upper bound is outside whatever its last bits; a remainder is
+// zero (+0 on both paths, a being positive) or a multiple of half an ulp of h,
+// hence at least 2^-64. Anything else (a start on the grid's lower faces, a
+// position that left through one) takes the guarded divisions.
+//
+// The floor and its integer come from one round-down add: for 0 <= q < 2^23,
+// RD(q + 2^23) is 2^23 + floor(q), whose low mantissa bits are floor(q), and
+// subtracting 2^23 again is exact. Inside the grid q < n - 1 <= 2^23 (the
+// field's axes hold at most 2^23 nodes); outside it neither value is used.
+__device__ __forceinline__ void floor_bits(const float q[3], float s[3], Cell& c) {
+  constexpr uint32_t kTwo23 = 0x4B000000u;  // the bits of 2^23
+  uint32_t i[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float b = __fadd_rd(q[k], 0x1p23f);
+    s[k] = __fsub_rn(b, 0x1p23f);
+    i[k] = __float_as_uint(b) - kTwo23;
+  }
+  c = {i[0], i[1], i[2]};
 }
 
-// Locates p; node receives the index of the cell's first corner within its
-// slice (meaningful only when p is inside).
+// Locates p; c receives its cell (meaningful only when p is inside).
 template <int kLocate>
-__device__ __forceinline__ bool locate(const FieldView& f, const Position& p, uint32_t& node,
+__device__ __forceinline__ bool locate(const FieldView& f, const Position& p, Cell& c,
                                        Weights& w) {
-  float q0, q2, q1;
-  float a0 = 0.0f;
-  float2 a21 = make_float2(0.0f, 0.0f);
+  const float x[3] = {p.p0, p.p21.y, p.p21.x};
+  float q[3], s[3], v[3];
   if constexpr (kLocate == kLocatePow2) {
     // q = p / h - offset / h in one rounding: p / h and offset / h are exact,
     // so this is the reference's rounded (p - offset) scaled by 1 / h.
-    q0 = __fmaf_rn(p.p0, f.reciprocal[0], -f.scaled_offset[0]);
-    const float2 q21 =
-        __ffma2_rn(p.p21, make_float2(f.reciprocal[2], f.reciprocal[1]),
-                   make_float2(-f.scaled_offset[2], -f.scaled_offset[1]));
-    q2 = q21.x;
-    q1 = q21.y;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) q[k] = __fmaf_rn(x[k], f.reciprocal[k], -f.scaled_offset[k]);
+    floor_bits(q, s, c);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = __fsub_rn(q[k], s[k]);
   } else {
-    a0 = __fsub_rn(p.p0, f.offset[0]);
-    a21 = sum2(p.p21, neg2(make_float2(f.offset[2], f.offset[1])));
-    if constexpr (kLocate == kLocateReciprocal) {
-      const float a[3] = {a0, a21.y, a21.x};
-      float q[3];
-      divide3_by_reciprocal(a, f.spacing, f.reciprocal, f.reciprocal_lo, q);
-      q0 = q[0];
-      q1 = q[1];
-      q2 = q[2];
+    float a[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = __fsub_rn(x[k], f.offset[k]);
+    if (kLocate == kLocateReciprocal && a[0] >= 0x1p-64f && a[1] >= 0x1p-64f &&
+        a[2] >= 0x1p-64f) {
+      auto divide = [&](float n, int k) {
+        return __fmaf_rn(n, f.reciprocal[k], __fmul_rn(n, f.reciprocal_lo[k]));
+      };
+#pragma unroll
+      for (int k = 0; k < 3; ++k) q[k] = divide(a[k], k);
+      floor_bits(q, s, c);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        float r = __fmaf_rn(-s[k], f.spacing[k], a[k]);
+        if (r < 0.0f) r = __fadd_rn(r, f.spacing[k]);
+        v[k] = divide(r, k);
+      }
     } else {
-      q0 = divide_spacing<kLocate>(a0, f.spacing[0], f.reciprocal[0], f.reciprocal_lo[0]);
-      q2 = divide_spacing<kLocate>(a21.x, f.spacing[2], f.reciprocal[2], f.reciprocal_lo[2]);
-      q1 = divide_spacing<kLocate>(a21.y, f.spacing[1], f.reciprocal[1], f.reciprocal_lo[1]);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        q[k] = divide_spacing<kLocate>(a[k], f.spacing[k], f.reciprocal[k], f.reciprocal_lo[k]);
+      floor_bits(q, s, c);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        v[k] = divide_spacing<kLocate>(remainder_general(a[k], s[k], f.spacing[k]), f.spacing[k],
+                                       f.reciprocal[k], f.reciprocal_lo[k]);
     }
   }
-  // floor(q) and its integer from one round-down add: for 0 <= q < 2^23,
-  // RD(q + 2^23) is 2^23 + floor(q), whose low mantissa bits are floor(q),
-  // and subtracting 2^23 again is exact. Inside the grid q < n - 1 <= 2^23
-  // (the field's axes hold at most 2^23 nodes); outside it neither value is
-  // used. (At q = -0 the floor is +0 instead of -0, which the weights' sign
-  // rules below undo.)
-  const float b0 = __fadd_rd(q0, 0x1p23f), b1 = __fadd_rd(q1, 0x1p23f),
-              b2 = __fadd_rd(q2, 0x1p23f);
-  const float s0 = __fsub_rn(b0, 0x1p23f), s1 = __fsub_rn(b1, 0x1p23f),
-              s2 = __fsub_rn(b2, 0x1p23f);
-  if constexpr (kLocate == kLocatePow2) {
-    w.w0 = copysignf(__fsub_rn(q0, s0), q0);
-    const float2 d = sum2(make_float2(q2, q1), neg2(make_float2(s2, s1)));
-    w.w21 = make_float2(copysignf(d.x, q2), copysignf(d.y, q1));
-  } else if constexpr (kLocate == kLocateReciprocal) {
-    const float a[3] = {a0, a21.y, a21.x};
-    const float s[3] = {s0, s1, s2};
-    float r[3], ww[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) r[i] = remainder_general(a[i], s[i], f.spacing[i]);
-    divide3_by_reciprocal(r, f.spacing, f.reciprocal, f.reciprocal_lo, ww);
-    w.w0 = ww[0];
-    w.w21 = make_float2(ww[2], ww[1]);
-  } else {
-    w.w0 = weight_general<kLocate>(a0, s0, f.spacing[0], f.reciprocal[0], f.reciprocal_lo[0]);
-    w.w21 = make_float2(
-        weight_general<kLocate>(a21.x, s2, f.spacing[2], f.reciprocal[2], f.reciprocal_lo[2]),
-        weight_general<kLocate>(a21.y, s1, f.spacing[1], f.reciprocal[1], f.reciprocal_lo[1]));
-  }
-  // The integer floors (the bits of b minus those of 2^23) decide inside:
+  w.w0 = v[0];
+  w.w21 = make_float2(v[2], v[1]);
   // 0 <= q < n - 1 iff 0 <= floor(q) < n - 1, and a negative, NaN, infinite
   // or too large q gives a difference of n - 1 or more as an unsigned value
   // (-0 gives 0, inside, as the reference has it).
-  constexpr uint32_t kTwo23 = 0x4B000000u;  // the bits of 2^23
-  const uint32_t i0 = __float_as_uint(b0), i1 = __float_as_uint(b1), i2 = __float_as_uint(b2);
-  const bool inside =
-      (i0 - kTwo23 < f.cells[0]) & (i1 - kTwo23 < f.cells[1]) & (i2 - kTwo23 < f.cells[2]);
-  node = i0 * f.stride0 + i1 * f.stride1 + i2 - f.node_bias;
-  return inside;
+  return (c.i0 < f.cells[0]) & (c.i1 < f.cells[1]) & (c.i2 < f.cells[2]);
 }
 
-// (1 - w) * lo + w * hi per lane, every operation rounded on its own.
-__device__ __forceinline__ float2 lerp2(float2 lo, float2 hi, float2 one_minus_w, float2 w) {
-  return add2(mul2(one_minus_w, lo), mul2(w, hi));
+// Index of a cell's first node within its slice.
+__device__ __forceinline__ uint32_t first_node(const FieldView& f, const Cell& c) {
+  return c.i0 * f.stride0 + c.i1 * f.stride1 + c.i2;
 }
 
 // The eight corners of one cell are corner j = dx * 4 + dy * 2 + dz (the
-// permute_for order of permute_for.hpp:12-34). Two register layouts of them
+// permute_for order of permute_for.hpp:12-34). Three register layouts of them
 // serve the trilinear reduction of regular_grid.hpp:71-73 (axis 2, then 1,
-// then 0, with c[j] = (1 - w) * c[2j] + w * c[2j+1]); both give the same
-// bits, and each storage takes the one that measured faster on the B200.
+// then 0, with c[j] = (1 - w) * c[2j] + w * c[2j+1]); all give the same bits,
+// and each storage takes the one that its loads fill without register moves.
 //
-// CornerNodes (F32 nodes): xy[j] = (v0, v1) of corner j, and the v2
-// components paired as (corner 0, corner 4), (1, 5), (2, 6), (3, 7). A
-// 16-byte node load lands (v0, v1) in a register pair as it is, and the
-// lerps multiply in scalar: packed products would need the weights
-// duplicated into pairs, and the extra registers cost more than the packed
-// multiply saves at F32's load width.
+// CornerNodes (F32 nodes): xy[j] = (v0, v1) of corner j as the 16-byte node
+// load leaves them, blended in packed form, and the third component beside
+// them in scalar form. (Scalar lerps throughout: 6.6e9 warp instructions
+// against 5.7e9 on a million seeds of 2000 steps; the launch, bound by the L1
+// data pipe there, takes 10.4 and 10.2 ms.)
 struct CornerNodes {
   float2 xy[8];
-  float2 z04, z15, z26, z37;
+  float z[8];
 };
 
-// CornerEdges (F16 / BF16 nodes, F32 edge records): z[e][c] = (component c
-// of corner 2e, component c of corner 2e + 1), the two ends of edge
-// e = dx * 2 + dy along axis 2, formed as 16-bit values are widened or loaded
-// as they are from an edge record. Each lerp is one packed multiply of
-// (lo, hi) by the weight pair (1 - w, w) and one scalar sum. (F32 nodes in
-// this layout, pairs formed by register moves after the loads, measured 5 %
-// slower on the headline launch than CornerNodes.)
+// CornerPairs (F16 / BF16 nodes): p[k][c] = (component c of corner k, of
+// corner k + 4), the two ends of an edge along axis 0, formed as 16-bit values
+// are widened. Blends along axes 2 and 1 are packed over the two ends; the
+// last, along axis 0, is one packed multiply and one scalar sum. (Pairs along
+// axis 2, one packed multiply and one scalar sum for each of the 21 lerps: 224
+// warp instructions a step against 202, 542 against 515 us a call of 200,003
+// seeds and 400 steps in a stream of calls.)
+struct CornerPairs {
+  float2 p[4][3];
+};
+
+// CornerEdges (F32 edge records): z[e][c] = (component c of corner 2e,
+// component c of corner 2e + 1), the two ends of edge e = dx * 2 + dy along
+// axis 2, loaded as they are from an edge record. Each lerp is one packed
+// multiply of (lo, hi) by the weight pair (1 - w, w) and one scalar sum.
 struct CornerEdges {
   float2 z[4][3];
 };
 
 template <int kStorage>
-using CornersOf = std::conditional_t<kStorage == DPA_STORAGE_F32, CornerNodes, CornerEdges>;
+using CornersOf = std::conditional_t<
+    kStorage == DPA_STORAGE_F32, CornerNodes,
+    std::conditional_t<kStorage == DPA_STORAGE_F32_EDGES, CornerEdges, CornerPairs>>;
 
 // Node layouts (F32, F16, BF16): one 16-byte float4 (F32) or 8-byte uint2
 // per node.
@@ -257,95 +265,77 @@ template <int kStorage>
 __device__ __forceinline__ void gather(const FieldView& f, uint32_t node, CornerNodes& k,
                                        int64_t slice_base = 0) {
   const CellEdges<kStorage> c(f, node, slice_base);
-  float z[8];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    load_node<kStorage>(c.e[e], 0, k.xy[2 * e].x, k.xy[2 * e].y, z[2 * e]);
-    load_node<kStorage>(c.e[e], 1, k.xy[2 * e + 1].x, k.xy[2 * e + 1].y, z[2 * e + 1]);
+    load_node<kStorage>(c.e[e], 0, k.xy[2 * e].x, k.xy[2 * e].y, k.z[2 * e]);
+    load_node<kStorage>(c.e[e], 1, k.xy[2 * e + 1].x, k.xy[2 * e + 1].y, k.z[2 * e + 1]);
   }
-  k.z04 = make_float2(z[0], z[4]);
-  k.z15 = make_float2(z[1], z[5]);
-  k.z26 = make_float2(z[2], z[6]);
-  k.z37 = make_float2(z[3], z[7]);
 }
 
 // gather() of F32 nodes into CornerNodes only where `need` holds, by
 // predicated loads instead of a branch: elsewhere the corners keep their
 // values and no load is made.
-__device__ __forceinline__ void load_node_if(bool need, const float4* at, float& x, float& y,
-                                             float& z) {
-  float w = 0.0f;
-  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t"
-      "@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-      : "+f"(x), "+f"(y), "+f"(z), "+f"(w)
+__device__ __forceinline__ void load_node_if(bool need, const float4* at, float2& xy, float& z) {
+  asm("{\n\t.reg .pred p;\n\t.reg .f32 pad;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+      "@p ld.global.nc.v4.f32 {%0, %1, %2, pad}, [%3];\n\t}"
+      : "+f"(xy.x), "+f"(xy.y), "+f"(z)
       : "l"(at), "r"(need ? 1u : 0u));
 }
 
 __device__ __forceinline__ void gather_if(const FieldView& f, uint32_t node, bool need,
                                           CornerNodes& k) {
   const CellEdges<DPA_STORAGE_F32> c(f, node, 0);
-  float z[8] = {k.z04.x, k.z15.x, k.z26.x, k.z37.x, k.z04.y, k.z15.y, k.z26.y, k.z37.y};
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    load_node_if(need, c.e[e], k.xy[2 * e].x, k.xy[2 * e].y, z[2 * e]);
-    load_node_if(need, c.e[e] + 1, k.xy[2 * e + 1].x, k.xy[2 * e + 1].y, z[2 * e + 1]);
+    load_node_if(need, c.e[e], k.xy[2 * e], k.z[2 * e]);
+    load_node_if(need, c.e[e] + 1, k.xy[2 * e + 1], k.z[2 * e + 1]);
   }
-  k.z04 = make_float2(z[0], z[4]);
-  k.z15 = make_float2(z[1], z[5]);
-  k.z26 = make_float2(z[2], z[6]);
-  k.z37 = make_float2(z[3], z[7]);
+}
+
+template <int kStorage>
+__device__ __forceinline__ void gather(const FieldView& f, uint32_t node, CornerPairs& k,
+                                       int64_t slice_base = 0) {
+  const CellEdges<kStorage> c(f, node, slice_base);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a[3], b[3];
+    load_node<kStorage>(c.e[j >> 1], j & 1, a[0], a[1], a[2]);
+    load_node<kStorage>(c.e[2 + (j >> 1)], j & 1, b[0], b[1], b[2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) k.p[j][i] = make_float2(a[i], b[i]);
+  }
 }
 
 template <int kStorage>
 __device__ __forceinline__ void gather(const FieldView& f, uint32_t node, CornerEdges& k,
                                        int64_t slice_base = 0) {
-  if constexpr (kStorage == DPA_STORAGE_F32_EDGES) {
-    const char* base = static_cast<const char*>(f.nodes) +
-                       (uint64_t(slice_base) + node) * uint64_t(kEdgeRecordBytes);
-    const uint64_t s1 = uint64_t(f.stride1) * kEdgeRecordBytes;
-    const uint64_t s0 = uint64_t(f.stride0) * kEdgeRecordBytes;
-    load_edge_record(base, k.z[0]);
-    load_edge_record(base + s1, k.z[1]);
-    load_edge_record(base + s0, k.z[2]);
-    load_edge_record(base + s0 + s1, k.z[3]);
-  } else {
-    const CellEdges<kStorage> c(f, node, slice_base);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float lo[3], hi[3];
-      load_node<kStorage>(c.e[e], 0, lo[0], lo[1], lo[2]);
-      load_node<kStorage>(c.e[e], 1, hi[0], hi[1], hi[2]);
-#pragma unroll
-      for (int c2 = 0; c2 < 3; ++c2) k.z[e][c2] = make_float2(lo[c2], hi[c2]);
-    }
-  }
+  const char* base = static_cast<const char*>(f.nodes) +
+                     (uint64_t(slice_base) + node) * uint64_t(kEdgeRecordBytes);
+  const uint64_t s1 = uint64_t(f.stride1) * kEdgeRecordBytes;
+  const uint64_t s0 = uint64_t(f.stride0) * kEdgeRecordBytes;
+  load_edge_record(base, k.z[0]);
+  load_edge_record(base + s1, k.z[1]);
+  load_edge_record(base + s0, k.z[2]);
+  load_edge_record(base + s0 + s1, k.z[3]);
 }
 
-__device__ __forceinline__ void trilinear(const CornerNodes& k, const Weights& w, float2& v01,
-                                          float& v2) {
-  const float2 t21 = sum2(splat(1.0f), neg2(w.w21));
-  const float t0 = __fsub_rn(1.0f, w.w0);
-  const float2 W2 = splat(w.w21.x), T2 = splat(t21.x);
-  const float2 W1 = splat(w.w21.y), T1 = splat(t21.y);
-  const float2 W0 = splat(w.w0), T0 = splat(t0);
-  auto lerp = [](float2 lo, float2 hi, float2 t, float2 u) {
-#if DPA_F32_PACKED_LERP
-    return add2(mul2(t, lo), mul2(u, hi));
-#else
-    return add2(mul2_scalar(t, lo), mul2_scalar(u, hi));
-#endif
-  };
-  const float2 e0 = lerp(k.xy[0], k.xy[1], T2, W2);
-  const float2 e1 = lerp(k.xy[2], k.xy[3], T2, W2);
-  const float2 e2 = lerp(k.xy[4], k.xy[5], T2, W2);
-  const float2 e3 = lerp(k.xy[6], k.xy[7], T2, W2);
-  const float2 f0 = lerp(e0, e1, T1, W1);
-  const float2 f1 = lerp(e2, e3, T1, W1);
-  v01 = lerp(f0, f1, T0, W0);
-  const float2 e02 = lerp(k.z04, k.z15, T2, W2);  // (e0, e2) of component 2
-  const float2 e13 = lerp(k.z26, k.z37, T2, W2);  // (e1, e3)
-  const float2 f01 = lerp(e02, e13, T1, W1);      // (f0, f1)
-  v2 = __fadd_rn(__fmul_rn(t0, f01.x), __fmul_rn(w.w0, f01.y));
+__device__ __forceinline__ void trilinear(const FieldView& f, const CornerNodes& k,
+                                          const Weights& w, float2& v01, float& v2) {
+  const float2 unit = make_float2(f.unit[0], f.unit[1]);
+  const float w2 = w.w21.x, t2 = __fsub_rn(1.0f, w2);
+  const float w1 = w.w21.y, t1 = __fsub_rn(1.0f, w1);
+  const float w0 = w.w0, t0 = __fsub_rn(1.0f, w0);
+  float2 e[4];
+  float z[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    e[r] = blend2(k.xy[2 * r], k.xy[2 * r + 1], splat(t2), splat(w2), unit);
+    z[r] = blend(k.z[2 * r], k.z[2 * r + 1], t2, w2);
+  }
+  const float2 f0 = blend2(e[0], e[1], splat(t1), splat(w1), unit);
+  const float2 f1 = blend2(e[2], e[3], splat(t1), splat(w1), unit);
+  v01 = blend2(f0, f1, splat(t0), splat(w0), unit);
+  v2 = blend(blend(z[0], z[1], t1, w1), blend(z[2], z[3], t1, w1), t0, w0);
 }
 
 // (1 - w) * lo + w * hi for the pair lohi = (lo, hi) and tw = (1 - w, w).
@@ -354,8 +344,25 @@ __device__ __forceinline__ float lerp_pair(float2 lohi, float2 tw) {
   return __fadd_rn(m.x, m.y);
 }
 
-__device__ __forceinline__ void trilinear(const CornerEdges& k, const Weights& w, float2& v01,
-                                          float& v2) {
+__device__ __forceinline__ void trilinear(const FieldView& f, const CornerPairs& k,
+                                          const Weights& w, float2& v01, float& v2) {
+  const float2 unit = make_float2(f.unit[0], f.unit[1]);
+  const float2 w2 = splat(w.w21.x), t2 = splat(__fsub_rn(1.0f, w.w21.x));
+  const float2 w1 = splat(w.w21.y), t1 = splat(__fsub_rn(1.0f, w.w21.y));
+  const float2 tw0 = make_float2(__fsub_rn(1.0f, w.w0), w.w0);
+  float v[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float2 e0 = blend2(k.p[0][i], k.p[1][i], t2, w2, unit);
+    const float2 e1 = blend2(k.p[2][i], k.p[3][i], t2, w2, unit);
+    v[i] = lerp_pair(blend2(e0, e1, t1, w1, unit), tw0);
+  }
+  v01 = make_float2(v[0], v[1]);
+  v2 = v[2];
+}
+
+__device__ __forceinline__ void trilinear(const FieldView&, const CornerEdges& k,
+                                          const Weights& w, float2& v01, float& v2) {
   const float2 tw2 = make_float2(__fsub_rn(1.0f, w.w21.x), w.w21.x);
   const float2 tw1 = make_float2(__fsub_rn(1.0f, w.w21.y), w.w21.y);
   const float2 tw0 = make_float2(__fsub_rn(1.0f, w.w0), w.w0);
@@ -385,14 +392,15 @@ struct CellSampler {
   // and v2.
   __device__ __forceinline__ bool sample(const FieldView& f, const Position& p, float /*t*/,
                                          float2& v01, float& v2) {
-    uint32_t node;
+    Cell c;
     Weights w;
-    if (!locate<kLocate>(f, p, node, w)) return false;
+    if (!locate<kLocate>(f, p, c, w)) return false;
+    const uint32_t node = first_node(f, c);
     if (node != cached) {
       gather<kStorage>(f, node, corners);
       cached = node;
     }
-    trilinear(corners, w, v01, v2);
+    trilinear(f, corners, w, v01, v2);
     return true;
   }
 
@@ -401,9 +409,10 @@ struct CellSampler {
   // ones) is to be discarded.
   __device__ __forceinline__ bool sample_selected(const FieldView& f, const Position& p,
                                                   float2& v01, float& v2) {
-    uint32_t node;
+    Cell c;
     Weights w;
-    const bool inside = locate<kLocate>(f, p, node, w);
+    const bool inside = locate<kLocate>(f, p, c, w);
+    const uint32_t node = first_node(f, c);
     const bool need = inside && node != cached;
     if constexpr (kStorage == DPA_STORAGE_F32) {
       gather_if(f, node, need, corners);
@@ -412,11 +421,13 @@ struct CellSampler {
       gather<kStorage>(f, node, corners);
       cached = node;
     }
-    trilinear(corners, w, v01, v2);
+    trilinear(f, corners, w, v01, v2);
     return inside;
   }
 
   static constexpr bool kSteady = true;
+  // (An edge-record field's kernels are at their register limit.)
+  static constexpr bool kPackedSums = kStorage != DPA_STORAGE_F32_EDGES;
 
   __device__ __forceinline__ void reset() { cached = ~0u; }
 };
@@ -437,7 +448,7 @@ __device__ __forceinline__ bool locate_time(const FieldView& f, float t, int64_t
   if (r == 0.0f) r = copysignf(0.0f, a);
   w = f.time_fast ? divide_by_reciprocal(r, f.time_spacing, y, yl)
                    : __fdiv_rn(r, f.time_spacing);
-  slice_base = int64_t(s) * f.slice_stride;
+  slice_base = int64_t(uint64_t(uint32_t(s)) * uint64_t(f.slice_stride));
   return true;
 }
 
@@ -455,9 +466,10 @@ struct TimeSampler {
 
   __device__ __forceinline__ bool sample(const FieldView& f, const Position& p, float t,
                                          float2& v01, float& v2) {
-    uint32_t node;
+    Cell c;
     Weights w;
-    if (!locate<kLocate>(f, p, node, w)) return false;
+    if (!locate<kLocate>(f, p, c, w)) return false;
+    const uint32_t node = first_node(f, c);
     int64_t slice = 0;
     float wt = 0.0f;
     if (!locate_time(f, t, slice, wt)) return false;
@@ -469,15 +481,16 @@ struct TimeSampler {
     }
     float2 a01, b01;
     float a2, b2;
-    trilinear(lo, w, a01, a2);
-    trilinear(hi, w, b01, b2);
+    trilinear(f, lo, w, a01, a2);
+    trilinear(f, hi, w, b01, b2);
     const float u = __fsub_rn(1.0f, wt);
-    v01 = add2(mul2_scalar(splat(u), a01), mul2_scalar(splat(wt), b01));
-    v2 = __fadd_rn(__fmul_rn(u, a2), __fmul_rn(wt, b2));
+    v01 = blend2(a01, b01, splat(u), splat(wt), make_float2(f.unit[0], f.unit[1]));
+    v2 = blend(a2, b2, u, wt);
     return true;
   }
 
   static constexpr bool kSteady = false;
+  static constexpr bool kPackedSums = true;
 
   __device__ __forceinline__ void reset() {
     cached = ~0u;
@@ -559,6 +572,14 @@ __device__ __forceinline__ void general_step(const GeneralCoefficients& g, float
   h.started = true;
 }
 
+// a + b for the sum of a position and a product: packed (add2), or for
+// samplers that hold no unit pair two scalar sums.
+template <bool kPacked>
+__device__ __forceinline__ float2 advance(float2 a, float2 b, float2 unit) {
+  if constexpr (kPacked) return add2(a, b, unit);
+  else return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+
 // One integrator step in place. The derivative of p0 is v2 and that of
 // (p2, p1) is (v0, v1) (particle_advector.cpp:369).
 // t is the particle's time (used by time-varying fields only); the caller
@@ -569,6 +590,7 @@ template <int kIntegrator, class Sampler>
 __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& k,
                                    Sampler& sampler, Position& p, float t,
                                    StepHistory& history, bool active = true) {
+  const float2 unit = make_float2(f.unit[0], f.unit[1]);
   float2 v01;
   float v2;
   if constexpr (Sampler::kSteady && (kIntegrator == DPA_INTEGRATOR_EULER ||
@@ -582,12 +604,12 @@ __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& 
     Position n = p;
     if constexpr (kIntegrator == DPA_INTEGRATOR_EULER) {
       n.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, v2));
-      n.p21 = add2(p.p21, mul2(splat(k.dt), v01));
+      n.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.dt), v01), unit);
     } else {
       const float m0 = __fmul_rn(k.c0, v2), m1 = __fmul_rn(k.c1, v2);
       n.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, m0), m1), m1), m0);
       const float2 n0 = mul2(splat(k.c0), v01), n1 = mul2(splat(k.c1), v01);
-      n.p21 = add2(add2(add2(add2(p.p21, n0), n1), n1), n0);
+      n.p21 = advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(p.p21, n0, unit), n1, unit), n1, unit), n0, unit);
     }
     const bool taken = active && inside && !zero;
     p.p0 = taken ? n.p0 : p.p0;
@@ -601,14 +623,14 @@ __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& 
   if constexpr (kIntegrator == DPA_INTEGRATOR_EULER) {
     // odeint euler: x = 1 * x + dt * dxdt
     p.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, v2));
-    p.p21 = add2(p.p21, mul2(splat(k.dt), v01));
+    p.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.dt), v01), unit);
   } else if constexpr (kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4) {
     // odeint runge_kutta4, final stage with four equal stage derivatives:
     // x = 1 * x + (b0 dt) d + (b1 dt) d + (b2 dt) d + (b3 dt) d, left to right.
     const float m0 = __fmul_rn(k.c0, v2), m1 = __fmul_rn(k.c1, v2);
     p.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, m0), m1), m1), m0);
     const float2 n0 = mul2(splat(k.c0), v01), n1 = mul2(splat(k.c1), v01);
-    p.p21 = add2(add2(add2(add2(p.p21, n0), n1), n1), n0);
+    p.p21 = advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(p.p21, n0, unit), n1, unit), n1, unit), n0, unit);
   } else if constexpr (kIntegrator == kGeneralIntegrator) {
     general_step(k.g, v01, v2, history, p);
   } else {
@@ -618,22 +640,23 @@ __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& 
     float k2_2, k3_2, k4_2;
     Position x;
     x.p0 = __fadd_rn(p.p0, __fmul_rn(k.half, v2));
-    x.p21 = add2(p.p21, mul2(splat(k.half), v01));
+    x.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.half), v01), unit);
     const float t_half = __fadd_rn(t, k.half), t_end = __fadd_rn(t, k.dt);
     if (!sampler.sample(f, x, t_half, k2_01, k2_2)) return kStepOutOfBounds;
     x.p0 = __fadd_rn(p.p0, __fmul_rn(k.half, k2_2));
-    x.p21 = add2(p.p21, mul2(splat(k.half), k2_01));
+    x.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.half), k2_01), unit);
     if (!sampler.sample(f, x, t_half, k3_01, k3_2)) return kStepOutOfBounds;
     x.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, k3_2));
-    x.p21 = add2(p.p21, mul2(splat(k.dt), k3_01));
+    x.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.dt), k3_01), unit);
     if (!sampler.sample(f, x, t_end, k4_01, k4_2)) return kStepOutOfBounds;
     p.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, __fmul_rn(k.c0, v2)),
                                          __fmul_rn(k.c1, k2_2)),
                                __fmul_rn(k.c1, k3_2)),
                      __fmul_rn(k.c0, k4_2));
     const float2 C0 = splat(k.c0), C1 = splat(k.c1);
-    p.p21 = add2(add2(add2(add2(p.p21, mul2(C0, v01)), mul2(C1, k2_01)), mul2(C1, k3_01)),
-                 mul2(C0, k4_01));
+    p.p21 = advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(p.p21, mul2(C0, v01), unit), mul2(C1, k2_01), unit),
+                      mul2(C1, k3_01), unit),
+                 mul2(C0, k4_01), unit);
   }
   return kStepTaken;
 }
