@@ -999,8 +999,8 @@ int dpa_ftle_estimate(dpa_context* ctx, const dpa_field* field, const float seed
     cudaStream_t s = ctx->stream;
     DPA_TRY_CUDA(ctx, ctx->ftle_original.reserve(count * 12));
     DPA_TRY_CUDA(ctx, ctx->ftle_final.reserve(count * 12));
-    DPA_TRY_CUDA(ctx, ctx->ftle_winners.reserve(cells * 8));
-    DPA_TRY_CUDA(ctx, ctx->ftle_flow.reserve(cells * 12));
+    if (mapping == DPA_FTLE_MAPPING_REFERENCE)
+      DPA_TRY_CUDA(ctx, ctx->ftle_winners.reserve(cells * 8));
     DPA_TRY_CUDA(ctx, ctx->ftle_out.reserve(cells * 4));
     if (count) {
       DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->ftle_original.ptr, original_positions, count * 12,
@@ -1010,8 +1010,7 @@ int dpa_ftle_estimate(dpa_context* ctx, const dpa_field* field, const float seed
     }
     a.original_positions = ctx->ftle_original.as<float>();
     a.final_positions = ctx->ftle_final.as<float>();
-    a.winners = ctx->ftle_winners.as<unsigned long long>();
-    a.flow = ctx->ftle_flow.as<float>();
+    a.winners = ctx->ftle_winners.ptr;
     a.ftle = ctx->ftle_out.as<float>();
     DPA_TRY_CUDA(ctx, dpa::launch_ftle(a, s));
     DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ftle, ctx->ftle_out.ptr, cells * 4, cudaMemcpyDeviceToHost, s));
@@ -1035,12 +1034,11 @@ int dpa_ftle_estimate_device(dpa_context* ctx, const dpa_field* field, const flo
                          shape_out, s, &a, &cells);
     if (st != DPA_OK || !device_ftle || cells == 0) return st;
     DPA_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    DPA_TRY_CUDA(ctx, ctx->ftle_winners.reserve(cells * 8));
-    DPA_TRY_CUDA(ctx, ctx->ftle_flow.reserve(cells * 12));
+    if (mapping == DPA_FTLE_MAPPING_REFERENCE)
+      DPA_TRY_CUDA(ctx, ctx->ftle_winners.reserve(cells * 8));
     a.original_positions = device_original_positions;
     a.final_positions = device_final_positions;
-    a.winners = ctx->ftle_winners.as<unsigned long long>();
-    a.flow = ctx->ftle_flow.as<float>();
+    a.winners = ctx->ftle_winners.ptr;
     a.ftle = device_ftle;
     DPA_TRY_CUDA(ctx, dpa::launch_ftle(a, s));
     return DPA_OK;

@@ -1,6 +1,8 @@
-// ftle.cu -- flow-map scatter, central-difference Jacobian, C = J^T J,
+// ftle.cu -- flow-map claims, central-difference Jacobian, C = J^T J,
 // FP64 largest eigenvalue and ln(sqrt(lambda)) / T per lattice cell
 // (ftle_estimator.cpp:7-65 with regular_grid::gradient, regular_grid.hpp:87-108).
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace dpa {
@@ -23,40 +25,35 @@ __device__ __forceinline__ bool reference_cell(const FtleArgs& a, uint64_t p, ui
   return true;
 }
 
-// Pass 1: every particle claims its cell; the largest particle index wins.
+// Reference mapping, first pass: every particle claims its cell; the largest
+// particle index wins. kIndex holds an index + 1 (0: nobody): 32 bits for all
+// but the largest counts, half the clearing and the atomics' traffic.
+template <class kIndex>
 __global__ void ftle_claim_kernel(const FtleArgs a) {
   const uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (p >= a.count) return;
   uint64_t cell;
-  if (reference_cell(a, p, cell)) atomicMax(a.winners + cell, (unsigned long long)(p + 1));
+  if (reference_cell(a, p, cell)) atomicMax(static_cast<kIndex*>(a.winners) + cell, kIndex(p + 1));
 }
 
-// Pass 2: the flow map holds the winner's final position, zero where no
-// particle landed (the reference's zero-initialized multi_array).
-__global__ void ftle_fill_kernel(const FtleArgs a, uint64_t cells) {
-  const uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= cells) return;
-  float x = 0.0f, y = 0.0f, z = 0.0f;
-  if (a.mapping == DPA_FTLE_MAPPING_LATTICE) {
-    x = a.final_positions[3 * c];
-    y = a.final_positions[3 * c + 1];
-    z = a.final_positions[3 * c + 2];
-  } else {
-    const unsigned long long w = a.winners[c];
-    if (w) {
-      const uint64_t p = w - 1;
-      x = a.final_positions[3 * p];
-      y = a.final_positions[3 * p + 1];
-      z = a.final_positions[3 * p + 2];
-    }
+// The flow map at a cell: the particle of that index (lattice mapping, kIndex
+// void), or the winner's final position, zero where no particle landed (the
+// reference's zero-initialized multi_array).
+template <class kIndex>
+__device__ __forceinline__ void flow_at(const FtleArgs& a, uint64_t cell, float v[3]) {
+  const float* at = a.final_positions + 3 * cell;
+  if constexpr (!std::is_void_v<kIndex>) {
+    const kIndex w = static_cast<const kIndex*>(a.winners)[cell];
+    v[0] = v[1] = v[2] = 0.0f;
+    if (!w) return;
+    at = a.final_positions + 3 * uint64_t(w - 1);
   }
-  a.flow[3 * c] = x;
-  a.flow[3 * c + 1] = y;
-  a.flow[3 * c + 2] = z;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) v[r] = at[r];
 }
 
 // Largest eigenvalue of a symmetric 3x3 matrix by cyclic Jacobi rotations.
-__device__ double max_eigenvalue(double a[3][3]) {
+__device__ __noinline__ double max_eigenvalue_jacobi(double a[3][3]) {
   for (int sweep = 0; sweep < 32; ++sweep) {
     const double off = a[0][1] * a[0][1] + a[0][2] * a[0][2] + a[1][2] * a[1][2];
     const double diag = a[0][0] * a[0][0] + a[1][1] * a[1][1] + a[2][2] * a[2][2];
@@ -89,34 +86,101 @@ __device__ double max_eigenvalue(double a[3][3]) {
   return fmax(a[0][0], fmax(a[1][1], a[2][2]));
 }
 
-// Pass 3: per lattice cell. J[r][d] = (flow[next_d] - flow[prev_d])[r] / (2 h_d)
-// with prev/next clamped at the border while the divisor stays 2 h_d.
-// C = J^T J in FP32 (Eigen's 3x3 lazy product, c0 + (c1 + c2)); the
-// eigenvalue and the logarithm in FP64.
-__global__ void ftle_kernel(const FtleArgs a, uint64_t cells) {
+// Largest eigenvalue of a symmetric 3x3 matrix from its characteristic cubic
+// (Smith, "Eigenvalues of a symmetric 3 x 3 matrix", Comm. ACM 4(4), 1961):
+// with q the mean of the diagonal, B = A - q I, p^2 = |B|^2 / 6 and
+// r = det(B) / (2 p^3), the eigenvalues are q + p x for the roots x of
+// x^3 - 3 x = 2 r. For r >= 0 the largest root lies apart, in [sqrt 3, 2], where
+// the cubic's slope is at least 6. It is found by Newton steps, two in 32 bits
+// from the chord of [sqrt 3, 2] (1e-7) and two in 64 with the 32-bit slope, which
+// leave rounding errors only. For r < 0 that root is the smallest eigenvalue's, with
+// its sign changed, and the largest is -x / 2 away from it plus half the gap of
+// the other two, sqrt(3 - 3/4 x^2). The gap loses digits as it closes:
+// 1 + r = 1e-8 leaves a relative error of 4e-12 in the eigenvalue, far below the
+// 6e-8 of the 32-bit result. Closer than that (a double largest eigenvalue) and
+// for matrices that are not finite the Jacobi rotations answer.
+//
+// The rotations throughout took 1900 warp instructions for 32 cells, 800 of them in
+// 64 bits: 132 us for 1.5 million cells at 70 % of the issue slots; this takes 480
+// and 32 us.
+__device__ __forceinline__ double max_eigenvalue(double a[3][3]) {
+  const double q = (a[0][0] + a[1][1] + a[2][2]) * (1.0 / 3.0);
+  const double b0 = a[0][0] - q, b1 = a[1][1] - q, b2 = a[2][2] - q;
+  const double u = a[0][1], v = a[0][2], w = a[1][2];
+  const double p2 = (b0 * b0 + b1 * b1 + b2 * b2 + 2.0 * (u * u + v * v + w * w)) * (1.0 / 6.0);
+  if (p2 == 0.0) return q;
+  const double inverse = rsqrt(p2), p = p2 * inverse;
+  const double half_det =
+      0.5 * (b0 * (b1 * b2 - w * w) - u * (u * b2 - w * v) + v * (u * w - b1 * v));
+  const double r = half_det * inverse * inverse * inverse;
+  if (!(r >= -1.0 + 1e-8) || !(p2 < 1e300)) return max_eigenvalue_jacobi(a);
+  const double two_r = fmin(2.0 * fabs(r), 2.0);
+  constexpr float kRoot3 = 1.7320508f;
+  float x0 = fmaf(0.5f * (2.0f - kRoot3), float(two_r), kRoot3);
+  float slope = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    slope = __fdividef(1.0f, fmaf(3.0f * x0, x0, -3.0f));
+    x0 -= fmaf(fmaf(x0, x0, -3.0f), x0, -float(two_r)) * slope;
+  }
+  double x = x0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) x -= fma(fma(x, x, -3.0), x, -two_r) * double(slope);
+  if (r < 0.0) x = 0.5 * x + sqrt(fmax(fma(-0.75 * x, x, 3.0), 0.0));
+  return fma(p, x, q);
+}
+
+// Per lattice cell: J[r][d] = (flow[next_d] - flow[prev_d])[r] / (2 h_d) with
+// prev/next clamped at the border while the divisor stays 2 h_d; C = J^T J in
+// FP32 (Eigen's 3x3 lazy product, c0 + (c1 + c2)); the eigenvalue and the
+// logarithm in FP64. kSize holds a cell index: 32-bit divisions unless the
+// lattice needs more. The neighbours come straight from the particles' final
+// positions (a pass that laid the flow map out first took 9 to 14 us more).
+template <class kIndex, class kSize>
+__global__ void __launch_bounds__(128) ftle_kernel(const FtleArgs a, uint64_t cells) {
   const uint64_t flat = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (flat >= cells) return;
-  const uint64_t n1n2 = a.shape[1] * a.shape[2];
-  uint64_t sub[3] = {flat / n1n2, (flat / a.shape[2]) % a.shape[1], flat % a.shape[2]};
-  const uint64_t step[3] = {n1n2, a.shape[2], 1};
+  const kSize n[3] = {kSize(a.shape[0]), kSize(a.shape[1]), kSize(a.shape[2])};
+  const kSize row = kSize(flat) / n[2];
+  const kSize sub[3] = {row / n[1], row % n[1], kSize(flat) - row * n[2]};
+  const uint64_t step[3] = {a.shape[1] * a.shape[2], a.shape[2], 1};
   float J[3][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const uint64_t prev = sub[d] > 0 ? flat - step[d] : flat;
-    const uint64_t next = sub[d] + 1 < a.shape[d] ? flat + step[d] : flat;
+    float prev[3], next[3];
+    flow_at<kIndex>(a, sub[d] > 0 ? flat - step[d] : flat, prev);
+    flow_at<kIndex>(a, sub[d] + 1 < n[d] ? flat + step[d] : flat, next);
 #pragma unroll
     for (int r = 0; r < 3; ++r)
-      J[r][d] = __fdiv_rn(__fsub_rn(a.flow[3 * next + r], a.flow[3 * prev + r]), a.two_spacing[d]);
+      J[r][d] = __fdiv_rn(__fsub_rn(next[r], prev[r]), a.two_spacing[d]);
   }
   double C[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      C[i][j] = double(__fadd_rn(__fmul_rn(J[0][i], J[0][j]),
-                                 __fadd_rn(__fmul_rn(J[1][i], J[1][j]), __fmul_rn(J[2][i], J[2][j]))));
-  const double lambda = max_eigenvalue(C);
-  a.ftle[flat] = float(log(sqrt(lambda)) / a.horizon);
+    for (int j = i; j < 3; ++j)
+      C[i][j] = C[j][i] =
+          double(__fadd_rn(__fmul_rn(J[0][i], J[0][j]),
+                           __fadd_rn(__fmul_rn(J[1][i], J[1][j]), __fmul_rn(J[2][i], J[2][j]))));
+  a.ftle[flat] = float(0.5 * log(max_eigenvalue(C)) * a.inverse_horizon);
+}
+
+template <class kIndex>
+cudaError_t launch_ftle_cells(const FtleArgs& a, uint64_t cells, cudaStream_t stream) {
+  const unsigned blocks = blocks_for(cells, 128);
+  if (cells <= 0xffffffffull) ftle_kernel<kIndex, uint32_t><<<blocks, 128, 0, stream>>>(a, cells);
+  else ftle_kernel<kIndex, uint64_t><<<blocks, 128, 0, stream>>>(a, cells);
+  return cudaGetLastError();
+}
+
+template <class kIndex>
+cudaError_t launch_ftle_claims(const FtleArgs& a, uint64_t cells, cudaStream_t stream) {
+  DPA_CUDA_TRY(cudaMemsetAsync(a.winners, 0, cells * sizeof(kIndex), stream));
+  if (a.count) {
+    ftle_claim_kernel<kIndex><<<blocks_for(a.count, 256), 256, 0, stream>>>(a);
+    DPA_CUDA_TRY(cudaGetLastError());
+  }
+  return launch_ftle_cells<kIndex>(a, cells, stream);
 }
 
 __global__ void lattice_kernel(float o0, float o1, float o2, float s0, float s1, float s2,
@@ -163,20 +227,14 @@ cudaError_t launch_random_seeds(const float offset[3], const float size[3], uint
   return cudaGetLastError();
 }
 
-cudaError_t launch_ftle(const FtleArgs& a, cudaStream_t stream) {
+cudaError_t launch_ftle(const FtleArgs& args, cudaStream_t stream) {
+  FtleArgs a = args;
+  a.inverse_horizon = 1.0 / a.horizon;
   const uint64_t cells = a.shape[0] * a.shape[1] * a.shape[2];
   if (cells == 0) return cudaSuccess;
-  if (a.mapping == DPA_FTLE_MAPPING_REFERENCE) {
-    DPA_CUDA_TRY(cudaMemsetAsync(a.winners, 0, cells * sizeof(unsigned long long), stream));
-    if (a.count) {
-      ftle_claim_kernel<<<blocks_for(a.count, 256), 256, 0, stream>>>(a);
-      DPA_CUDA_TRY(cudaGetLastError());
-    }
-  }
-  ftle_fill_kernel<<<blocks_for(cells, 256), 256, 0, stream>>>(a, cells);
-  DPA_CUDA_TRY(cudaGetLastError());
-  ftle_kernel<<<blocks_for(cells, 128), 128, 0, stream>>>(a, cells);
-  return cudaGetLastError();
+  if (a.mapping == DPA_FTLE_MAPPING_LATTICE) return launch_ftle_cells<void>(a, cells, stream);
+  return a.count < 0xffffffffull ? launch_ftle_claims<unsigned int>(a, cells, stream)
+                                 : launch_ftle_claims<unsigned long long>(a, cells, stream);
 }
 
 cudaError_t launch_lattice_seeds(const float offset[3], const float stride[3],

@@ -130,7 +130,7 @@ struct dpa_context {
   DeviceBuffer wide, vertex_offsets, segment_offsets, scan_temp, totals;
   DeviceBuffer out_vertices, out_colors, out_indices;
   PinnedBuffer host_vertices, host_colors, host_indices, host_totals, host_offsets;
-  DeviceBuffer ftle_winners, ftle_flow, ftle_out, ftle_original, ftle_final;
+  DeviceBuffer ftle_winners, ftle_out, ftle_original, ftle_final;
 
   void release_all() {
     scratch.release();
@@ -138,7 +138,7 @@ struct dpa_context {
                          &raw_counts,
                          &kept_vertices, &kept_segments, &wide, &vertex_offsets,
                          &segment_offsets, &scan_temp, &totals, &out_vertices, &out_colors,
-                         &out_indices, &ftle_winners, &ftle_flow, &ftle_out, &ftle_original,
+                         &out_indices, &ftle_winners, &ftle_out, &ftle_original,
                          &ftle_final};
     for (DeviceBuffer* b : d) b->release();
     PinnedBuffer* h[] = {&host_vertices, &host_colors, &host_indices, &host_totals,

@@ -194,8 +194,8 @@ struct FtleArgs {
   float spacing[3];        // field spacing * stride
   float two_spacing[3];
   double horizon;          // |step_size * iterations| as the reference rounds it
-  unsigned long long* winners;  // [cells], scratch
-  float* flow;             // [cells][3], scratch
+  double inverse_horizon;  // set by the launcher
+  void* winners;           // scratch of the reference mapping, 8 bytes a cell
   float* ftle;             // [cells]
 };
 

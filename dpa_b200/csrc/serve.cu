@@ -102,7 +102,7 @@ struct dpa_server {
   // Emission scratch.
   DeviceBuffer raw_counts, curve_totals, vertex_offsets, segment_offsets, scan_temp, out_vertices,
       out_colors, out_indices;
-  DeviceBuffer ftle_original, ftle_winners, ftle_flow, ftle_out;
+  DeviceBuffer ftle_original, ftle_winners, ftle_out;
   range_allocator slots, vertices;
   PinnedBuffer response_arena;
   range_allocator response_units;  // of response_arena, in kResponseUnit bytes
@@ -548,7 +548,6 @@ void dpa_server::finish(active_request& a, response_storage& out) {
   if (ftle && cells) {
     SERVER_TRY(ftle_original.reserve(n * 12));
     SERVER_TRY(ftle_winners.reserve(cells * 8));
-    SERVER_TRY(ftle_flow.reserve(cells * 12));
     SERVER_TRY(ftle_out.reserve(cells * 4));
     SERVER_TRY(cudaMemcpyAsync(ftle_original.ptr, a.p.positions.data(), n * 12,
                                cudaMemcpyHostToDevice, finish_stream));
@@ -557,8 +556,7 @@ void dpa_server::finish(active_request& a, response_storage& out) {
     f.final_positions = positions.as<float>() + 3 * first;
     f.mapping = DPA_FTLE_MAPPING_REFERENCE;
     f.horizon = double(std::fabs(q.step_size * float(q.iterations)));
-    f.winners = ftle_winners.as<unsigned long long>();
-    f.flow = ftle_flow.as<float>();
+    f.winners = ftle_winners.ptr;
     f.ftle = ftle_out.as<float>();
     SERVER_TRY(dpa::launch_ftle(f, finish_stream));
     SERVER_TRY(cudaMemcpyAsync(d + at[7], ftle_out.ptr, cells * 4, cudaMemcpyDeviceToHost,
