@@ -344,6 +344,8 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
       block, &resident, &sms)));
   if (a.count == 0) return cudaSuccess;  // nothing to do, or preparation only
   if (a.blocks_per_sm && int(a.blocks_per_sm) < resident) resident = int(a.blocks_per_sm);
+  if (!a.blocks_per_sm && f.threads_per_sm)
+    resident = std::min(resident, std::max(1, int(f.threads_per_sm / block)));
   const uint64_t needed = (lanes + block - 1) / block;
   const uint64_t blocks = std::min<uint64_t>(needed, uint64_t(resident) * uint64_t(sms));
   if (blocks == 0) return cudaSuccess;
@@ -364,18 +366,36 @@ cudaError_t launch_ppt(const FieldView& f, const AdvectArgs& a, cudaStream_t s) 
   return launch_typed<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, 1>(f, a, s);
 }
 
+template <int kIntegrator, int kStorage, int kMode, bool kUnsteady>
+cudaError_t launch_record(const FieldView& f, const AdvectArgs& a, bool record, cudaStream_t s) {
+  return record ? launch_ppt<kIntegrator, kStorage, kMode, true, kUnsteady>(f, a, s)
+                : launch_ppt<kIntegrator, kStorage, kMode, false, kUnsteady>(f, a, s);
+}
+
 template <int kIntegrator, int kStorage, bool kUnsteady>
 cudaError_t launch_locate(const FieldView& f, const AdvectArgs& a, bool record, cudaStream_t s) {
+  if constexpr (!kUnsteady) {
+    if (f.tiled) {
+      switch (f.locate) {
+        case kLocatePow2:
+          return launch_record<kIntegrator, kStorage, kLocatePow2 | kTiledBit, false>(f, a, record,
+                                                                                      s);
+        case kLocateReciprocal:
+          return launch_record<kIntegrator, kStorage, kLocateReciprocal | kTiledBit, false>(
+              f, a, record, s);
+        default:
+          return launch_record<kIntegrator, kStorage, kLocateDivide | kTiledBit, false>(
+              f, a, record, s);
+      }
+    }
+  }
   switch (f.locate) {
     case kLocatePow2:
-      return record ? launch_ppt<kIntegrator, kStorage, kLocatePow2, true, kUnsteady>(f, a, s)
-                    : launch_ppt<kIntegrator, kStorage, kLocatePow2, false, kUnsteady>(f, a, s);
+      return launch_record<kIntegrator, kStorage, kLocatePow2, kUnsteady>(f, a, record, s);
     case kLocateReciprocal:
-      return record ? launch_ppt<kIntegrator, kStorage, kLocateReciprocal, true, kUnsteady>(f, a, s)
-                    : launch_ppt<kIntegrator, kStorage, kLocateReciprocal, false, kUnsteady>(f, a, s);
+      return launch_record<kIntegrator, kStorage, kLocateReciprocal, kUnsteady>(f, a, record, s);
     default:
-      return record ? launch_ppt<kIntegrator, kStorage, kLocateDivide, true, kUnsteady>(f, a, s)
-                    : launch_ppt<kIntegrator, kStorage, kLocateDivide, false, kUnsteady>(f, a, s);
+      return launch_record<kIntegrator, kStorage, kLocateDivide, kUnsteady>(f, a, record, s);
   }
 }
 

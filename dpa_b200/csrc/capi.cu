@@ -599,7 +599,9 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     f->owner = ctx;
     f->storage = storage;
     const size_t node_bytes = dpa::field_node_bytes(storage);
-    cudaError_t e = f->nodes.reserve(nodes * node_bytes);
+    for (int i = 0; i < 3; ++i) f->view.n[i] = int32_t(shape[i]);
+    f->view.storage = storage;
+    cudaError_t e = f->nodes.reserve(dpa::choose_layout(f->view, slices) * node_bytes);
     const float* src = xyzv;
     DeviceBuffer staging;
     if (e == cudaSuccess && !device_input) {
@@ -609,7 +611,7 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
       src = staging.as<float>();
     }
     if (e == cudaSuccess)
-      e = dpa::launch_repack(src, nodes, uint32_t(shape[2]), storage, f->nodes.ptr, ctx->stream);
+      e = dpa::launch_repack(src, nodes, f->view, f->nodes.ptr, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     staging.release();
     if (e != cudaSuccess) {
@@ -627,7 +629,6 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     dpa::FieldView& v = f->view;
     v.nodes = f->nodes.ptr;
     for (int i = 0; i < 3; ++i) {
-      v.n[i] = int32_t(shape[i]);
       v.offset[i] = offset[i];
       v.spacing[i] = spacing[i];
       float hi = 0.0f, lo = 0.0f;
@@ -641,7 +642,6 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     v.stride0 = uint32_t(shape[1] * shape[2]);
     v.stride1 = uint32_t(shape[2]);
     v.unit[0] = v.unit[1] = 1.0f;
-    v.storage = storage;
     v.locate = dpa::kLocatePow2;
     if (!pow2 && ctx->ieee_division) {
       v.locate = dpa::kLocateDivide;

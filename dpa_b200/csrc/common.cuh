@@ -35,6 +35,22 @@ constexpr float kZeroPrecision = 1e-5f;
 //                      offset / h, and fmod(p - offset, h) / h = q - floor(q).
 enum LocateMode : int { kLocateDivide = 0, kLocateReciprocal = 1, kLocatePow2 = 2 };
 
+// Kernels of a tiled field are instantiated with this bit beside the mode.
+constexpr int kTiledBit = 4;
+
+// Node layout of large steady fields: tiles of about one 2 MiB page instead of
+// rows, so that the particles of an SM stay in few pages. Node (i0, i1, i2) of a
+// slice is at
+//   sum over axes of i * stride + (i / size) * jump   (stride 1 along axis 2),
+// the quotient i / size being the high word of i * magic (i < 2^23, size <= 64).
+// A tile's rows of nodes hold one node more than the tile, the next tile's first,
+// so that a cell's two nodes along axis 2 always follow each other.
+struct TileLayout {
+  uint32_t magic[3];
+  uint32_t stride[2];
+  uint32_t jump[3];
+};
+
 // Device view of a repacked field. Nodes are 4-wide (x, y, z, pad) so one
 // vector load fetches a node: float4 for F32, four 16-bit values for F16/BF16.
 // A slice holds fewer than 2^32 nodes, so a node's index within its slice is
@@ -51,6 +67,9 @@ struct FieldView {
   float scaled_offset[3];  // offset / spacing, exact; used by kLocatePow2 only
   float upper[3];          // n - 1: inside iff 0 <= (p - offset) / h < n - 1
   uint32_t cells[3];       // n - 1, the cells per axis
+  int32_t tiled;           // the nodes are in `tile` order
+  TileLayout tile;
+  uint32_t threads_per_sm; // the most a launch keeps resident by default (0: no limit)
   float unit[2];           // {1, 1}: a multiplier the compiler cannot see (sample.cuh)
   int32_t storage;         // dpa_storage
   // LocateMode of the spatial axes. kLocatePow2 needs every spacing a power

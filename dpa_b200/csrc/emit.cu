@@ -263,35 +263,54 @@ __global__ void __launch_bounds__(kScanThreads) offsets_tiles_kernel(
 // Node layouts: one float4 (F32) or (x, y, z, 0) half/bfloat quad per node.
 // F32_EDGES: record t holds nodes t and t + 1 along axis 2, each component's
 // pair side by side (sample.cuh); the last node of a row repeats itself, and
-// no cell reads that record's second half.
-template <int kStorage>
-__global__ void repack_kernel(const float* xyzv, uint64_t nodes, uint32_t n2, void* out) {
+// no cell reads that record's second half. In a tiled layout of nodes the first
+// node of a tile's row also ends the row of the tile before it.
+template <int kStorage, bool kTiled>
+__global__ void repack_kernel(const float* xyzv, uint64_t nodes, const FieldView f, void* out) {
   const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= nodes) return;
   const float x = xyzv[3 * t], y = xyzv[3 * t + 1], z = xyzv[3 * t + 2];
+  const uint32_t n2 = uint32_t(f.n[2]);
+  uint64_t at = t, copy = t;
+  if constexpr (kTiled) {  // one slice of fewer than 2^32 nodes
+    const uint32_t row = uint32_t(t) / n2, i2 = uint32_t(t) - row * n2;
+    const uint32_t i0 = row / uint32_t(f.n[1]), i1 = row - i0 * uint32_t(f.n[1]);
+    at = copy = tiled_node(f.tile, i0, i1, i2);
+    if (kStorage != DPA_STORAGE_F32_EDGES && i2 > 0 &&
+        __umulhi(i2, f.tile.magic[2]) != __umulhi(i2 - 1, f.tile.magic[2]))
+      copy = uint64_t(tiled_node(f.tile, i0, i1, i2 - 1)) + 1;
+  }
+  auto store = [&](auto* o, auto v) {
+    o[at] = v;
+    if (kTiled && copy != at) o[copy] = v;
+  };
   if constexpr (kStorage == DPA_STORAGE_F32_EDGES) {
     const uint64_t u = (t % n2) + 1 < n2 ? t + 1 : t;
-    float4* o = reinterpret_cast<float4*>(out) + 2 * t;
+    float4* o = reinterpret_cast<float4*>(out) + 2 * at;
     o[0] = make_float4(x, xyzv[3 * u], y, xyzv[3 * u + 1]);
     o[1] = make_float4(z, xyzv[3 * u + 2], 0.0f, 0.0f);
   } else if constexpr (kStorage == DPA_STORAGE_F32) {
-    (void)n2;
-    reinterpret_cast<float4*>(out)[t] = make_float4(x, y, z, 0.0f);
+    store(reinterpret_cast<float4*>(out), make_float4(x, y, z, 0.0f));
   } else if constexpr (kStorage == DPA_STORAGE_F16) {
     const __half2 a = __floats2half2_rn(x, y);
     const __half2 b = __floats2half2_rn(z, 0.0f);
-    uint2 r;
-    r.x = *reinterpret_cast<const unsigned*>(&a);
-    r.y = *reinterpret_cast<const unsigned*>(&b);
-    reinterpret_cast<uint2*>(out)[t] = r;
+    store(reinterpret_cast<uint2*>(out), make_uint2(*reinterpret_cast<const unsigned*>(&a),
+                                                    *reinterpret_cast<const unsigned*>(&b)));
   } else {
     const __nv_bfloat162 a = __floats2bfloat162_rn(x, y);
     const __nv_bfloat162 b = __floats2bfloat162_rn(z, 0.0f);
-    uint2 r;
-    r.x = *reinterpret_cast<const unsigned*>(&a);
-    r.y = *reinterpret_cast<const unsigned*>(&b);
-    reinterpret_cast<uint2*>(out)[t] = r;
+    store(reinterpret_cast<uint2*>(out), make_uint2(*reinterpret_cast<const unsigned*>(&a),
+                                                    *reinterpret_cast<const unsigned*>(&b)));
   }
+}
+
+template <int kStorage>
+cudaError_t launch_repack_as(const float* xyzv, uint64_t nodes, const FieldView& f, void* out,
+                             cudaStream_t stream) {
+  const unsigned grid = unsigned((nodes + 255) / 256);
+  if (f.tiled) repack_kernel<kStorage, true><<<grid, 256, 0, stream>>>(xyzv, nodes, f, out);
+  else repack_kernel<kStorage, false><<<grid, 256, 0, stream>>>(xyzv, nodes, f, out);
+  return cudaGetLastError();
 }
 
 inline unsigned blocks_for(uint64_t n, unsigned block) { return unsigned((n + block - 1) / block); }
@@ -345,26 +364,64 @@ uint64_t field_node_bytes(int storage) {
   return storage == DPA_STORAGE_F32_EDGES ? 32 : storage == DPA_STORAGE_F32 ? 16 : 8;
 }
 
-cudaError_t launch_repack(const float* xyzv, uint64_t nodes, uint32_t n2, int storage, void* out,
+cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& f, void* out,
                           cudaStream_t stream) {
   if (nodes == 0) return cudaSuccess;
-  const unsigned grid = blocks_for(nodes, 256);
-  switch (storage) {
-    case DPA_STORAGE_F32:
-      repack_kernel<DPA_STORAGE_F32><<<grid, 256, 0, stream>>>(xyzv, nodes, n2, out);
-      break;
-    case DPA_STORAGE_F16:
-      repack_kernel<DPA_STORAGE_F16><<<grid, 256, 0, stream>>>(xyzv, nodes, n2, out);
-      break;
-    case DPA_STORAGE_BF16:
-      repack_kernel<DPA_STORAGE_BF16><<<grid, 256, 0, stream>>>(xyzv, nodes, n2, out);
-      break;
+  switch (f.storage) {
+    case DPA_STORAGE_F32: return launch_repack_as<DPA_STORAGE_F32>(xyzv, nodes, f, out, stream);
+    case DPA_STORAGE_F16: return launch_repack_as<DPA_STORAGE_F16>(xyzv, nodes, f, out, stream);
+    case DPA_STORAGE_BF16: return launch_repack_as<DPA_STORAGE_BF16>(xyzv, nodes, f, out, stream);
     case DPA_STORAGE_F32_EDGES:
-      repack_kernel<DPA_STORAGE_F32_EDGES><<<grid, 256, 0, stream>>>(xyzv, nodes, n2, out);
-      break;
+      return launch_repack_as<DPA_STORAGE_F32_EDGES>(xyzv, nodes, f, out, stream);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+}
+
+// Where the lines lie, measured on curl noise with 2 million seeds of up to 1000
+// steps of a quarter cell (rows, tiles; threads per SM in brackets, ms):
+//   F32 320^3, 0.5 GB   9.0 [1024]             9.0 [1024]
+//   F32 400^3, 1.0 GB  20.8 [1024], 12.4 [512]  10.0 [1024]
+//   F32 512^3, 2.1 GB  29.1 [1024], 14.2 [512]  13.8 [1024], 11.9 [768], 14.2 [512]
+//   F32 768^3, 7.2 GB                           32.5 [1024], 16.8 [768], 17.0 [512]
+//   F16 512^3, 1.1 GB  15.9 [1024], 11.1 [768]  10.4 [1024], 11.3 [768]
+//   F16 768^3, 3.6 GB                           15.5 [1024], 13.6 [768]
+// Beyond about half a gigabyte the gathers of a full SM miss the address
+// translation cache: random 16-byte gathers fall from 2079 GB/s in a table of
+// 256 MB to 892 in one of 2 GB. Tiles keep a particle's path in fewer pages, and
+// fewer warps in flight leave room for their misses.
+uint64_t choose_layout(FieldView& v, uint32_t slices) {
+  constexpr uint64_t kTileBytes = 512ull << 20, kFewerThreadsBytes = 1280ull << 20;
+  const uint64_t node_bytes = field_node_bytes(v.storage);
+  const uint64_t nodes = uint64_t(v.n[0]) * uint64_t(v.n[1]) * uint64_t(v.n[2]);
+  v.tiled = 0;
+  v.tile = TileLayout{};
+  v.threads_per_sm = 0;
+  if (slices != 1 || nodes * node_bytes < kTileBytes) return nodes * slices;
+  // About 64 nodes an axis, of a 2 MiB page for F32 nodes (axis 2: 32); tiles of
+  // one axis are as even as they can be, so that little is allocated beyond the
+  // field.
+  const bool edges = v.storage == DPA_STORAGE_F32_EDGES;
+  const uint32_t want[3] = {64u, edges ? 32u : 64u, v.storage == DPA_STORAGE_F32 || edges ? 32u : 64u};
+  uint64_t size[3], tiles[3];
+  for (int i = 0; i < 3; ++i) {
+    tiles[i] = (uint64_t(v.n[i]) + want[i] - 1) / want[i];
+    size[i] = (uint64_t(v.n[i]) + tiles[i] - 1) / tiles[i];
+  }
+  const uint64_t row = size[2] + (edges ? 0 : 1);
+  const uint64_t tile = size[0] * size[1] * row;
+  const uint64_t total = tile * tiles[0] * tiles[1] * tiles[2];
+  v.threads_per_sm = 512;
+  // An axis of one node would need a magic of 2^32; the index is 32 bits wide.
+  if (size[0] < 2 || size[1] < 2 || size[2] < 2 || total >= (1ull << 32)) return nodes;
+  v.threads_per_sm = total * node_bytes > kFewerThreadsBytes ? 768 : 0;
+  v.tiled = 1;
+  for (int i = 0; i < 3; ++i) v.tile.magic[i] = uint32_t((1ull << 32) / size[i] + 1);
+  v.tile.stride[0] = uint32_t(size[1] * row);
+  v.tile.stride[1] = uint32_t(row);
+  v.tile.jump[0] = uint32_t(tiles[1] * tiles[2] * tile - size[0] * size[1] * row);
+  v.tile.jump[1] = uint32_t(tiles[2] * tile - size[1] * row);
+  v.tile.jump[2] = uint32_t(tile - size[2]);
+  return total;
 }
 
 }  // namespace dpa

@@ -178,11 +178,17 @@ cudaError_t launch_gather_probe(const float4* table, uint32_t mask, uint32_t sid
 cudaError_t launch_verify_division(float h, float y, float yl, unsigned int* mismatches,
                                    cudaStream_t stream);
 
-// Field repack: XYZV float [n][3] (rows of n2 nodes along axis 2) -> the
-// device layout of the given storage; field_node_bytes is its size per node.
+// Field repack: XYZV float [n][3] (rows of view.n[2] nodes along axis 2) -> the
+// device layout of view.storage and, when view.tiled, in view.tile's order;
+// field_node_bytes is its size per node.
 uint64_t field_node_bytes(int storage);
-cudaError_t launch_repack(const float* xyzv, uint64_t nodes, uint32_t n2, int storage, void* out,
+cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& view, void* out,
                           cudaStream_t stream);
+
+// The layout of a steady field of this shape and storage. Returns the nodes to
+// allocate; sets view.tiled, view.tile and view.threads_per_sm (view.n and
+// view.storage are set).
+uint64_t choose_layout(FieldView& view, uint32_t slices);
 
 struct FtleArgs {
   uint64_t count;

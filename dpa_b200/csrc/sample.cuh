@@ -179,9 +179,34 @@ __device__ __forceinline__ bool locate(const FieldView& f, const Position& p, Ce
   return (c.i0 < f.cells[0]) & (c.i1 < f.cells[1]) & (c.i2 < f.cells[2]);
 }
 
-// Index of a cell's first node within its slice.
-__device__ __forceinline__ uint32_t first_node(const FieldView& f, const Cell& c) {
-  return c.i0 * f.stride0 + c.i1 * f.stride1 + c.i2;
+// Index, within its slice, of a node in tile order.
+__device__ __forceinline__ uint32_t tiled_node(const TileLayout& t, uint32_t i0, uint32_t i1,
+                                               uint32_t i2) {
+  return i0 * t.stride[0] + __umulhi(i0, t.magic[0]) * t.jump[0] + i1 * t.stride[1] +
+         __umulhi(i1, t.magic[1]) * t.jump[1] + i2 + __umulhi(i2, t.magic[2]) * t.jump[2];
+}
+
+// Indices, within their slice, of the first nodes of a cell's four edges along
+// axis 2: e = dx * 2 + dy.
+struct CellRows {
+  uint32_t at[4];
+};
+
+template <bool kTiled>
+__device__ __forceinline__ CellRows cell_rows(const FieldView& f, const Cell& c) {
+  if constexpr (kTiled) {
+    const TileLayout& t = f.tile;
+    auto along = [&](int axis, uint32_t i) {
+      return i * t.stride[axis] + __umulhi(i, t.magic[axis]) * t.jump[axis];
+    };
+    const uint32_t a0 = along(0, c.i0), a1 = along(0, c.i0 + 1);
+    const uint32_t z = c.i2 + __umulhi(c.i2, t.magic[2]) * t.jump[2];
+    const uint32_t b0 = along(1, c.i1) + z, b1 = along(1, c.i1 + 1) + z;
+    return {a0 + b0, a0 + b1, a1 + b0, a1 + b1};
+  } else {
+    const uint32_t n = c.i0 * f.stride0 + c.i1 * f.stride1 + c.i2;
+    return {n, n + f.stride1, n + f.stride0, n + f.stride0 + f.stride1};
+  }
 }
 
 // The eight corners of one cell are corner j = dx * 4 + dy * 2 + dz (the
@@ -229,21 +254,6 @@ using CornersOf = std::conditional_t<
 template <int kStorage>
 using NodeOf = std::conditional_t<kStorage == DPA_STORAGE_F32, float4, uint2>;
 
-// Pointers to the first node of the cell's four edges along axis 2 (corners
-// 2e and 2e + 1 are consecutive nodes): e = dx * 2 + dy.
-template <int kStorage>
-struct CellEdges {
-  const NodeOf<kStorage>* e[4];
-  __device__ __forceinline__ CellEdges(const FieldView& f, uint32_t node, int64_t slice_base) {
-    const NodeOf<kStorage>* base =
-        reinterpret_cast<const NodeOf<kStorage>*>(f.nodes) + slice_base + node;
-    e[0] = base;
-    e[1] = base + f.stride1;
-    e[2] = base + f.stride0;
-    e[3] = e[2] + f.stride1;
-  }
-};
-
 // Edge records (F32_EDGES): record n holds node n and node n + 1 along axis
 // 2 with each component's two values side by side, (x_n, x_n+1, y_n, y_n+1,
 // z_n, z_n+1, 0, 0), 32 bytes read by one 256-bit load whose registers are
@@ -262,13 +272,19 @@ __device__ __forceinline__ void load_edge_record(const char* record, float2 out[
 }
 
 template <int kStorage>
-__device__ __forceinline__ void gather(const FieldView& f, uint32_t node, CornerNodes& k,
+__device__ __forceinline__ const NodeOf<kStorage>* row_pointer(const FieldView& f, uint32_t row,
+                                                               int64_t slice_base) {
+  return reinterpret_cast<const NodeOf<kStorage>*>(f.nodes) + slice_base + row;
+}
+
+template <int kStorage>
+__device__ __forceinline__ void gather(const FieldView& f, const CellRows& rows, CornerNodes& k,
                                        int64_t slice_base = 0) {
-  const CellEdges<kStorage> c(f, node, slice_base);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    load_node<kStorage>(c.e[e], 0, k.xy[2 * e].x, k.xy[2 * e].y, k.z[2 * e]);
-    load_node<kStorage>(c.e[e], 1, k.xy[2 * e + 1].x, k.xy[2 * e + 1].y, k.z[2 * e + 1]);
+    const NodeOf<kStorage>* at = row_pointer<kStorage>(f, rows.at[e], slice_base);
+    load_node<kStorage>(at, 0, k.xy[2 * e].x, k.xy[2 * e].y, k.z[2 * e]);
+    load_node<kStorage>(at, 1, k.xy[2 * e + 1].x, k.xy[2 * e + 1].y, k.z[2 * e + 1]);
   }
 }
 
@@ -282,41 +298,40 @@ __device__ __forceinline__ void load_node_if(bool need, const float4* at, float2
       : "l"(at), "r"(need ? 1u : 0u));
 }
 
-__device__ __forceinline__ void gather_if(const FieldView& f, uint32_t node, bool need,
+__device__ __forceinline__ void gather_if(const FieldView& f, const CellRows& rows, bool need,
                                           CornerNodes& k) {
-  const CellEdges<DPA_STORAGE_F32> c(f, node, 0);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    load_node_if(need, c.e[e], k.xy[2 * e], k.z[2 * e]);
-    load_node_if(need, c.e[e] + 1, k.xy[2 * e + 1], k.z[2 * e + 1]);
+    const float4* at = row_pointer<DPA_STORAGE_F32>(f, rows.at[e], 0);
+    load_node_if(need, at, k.xy[2 * e], k.z[2 * e]);
+    load_node_if(need, at + 1, k.xy[2 * e + 1], k.z[2 * e + 1]);
   }
 }
 
 template <int kStorage>
-__device__ __forceinline__ void gather(const FieldView& f, uint32_t node, CornerPairs& k,
+__device__ __forceinline__ void gather(const FieldView& f, const CellRows& rows, CornerPairs& k,
                                        int64_t slice_base = 0) {
-  const CellEdges<kStorage> c(f, node, slice_base);
+  const NodeOf<kStorage>* at[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) at[e] = row_pointer<kStorage>(f, rows.at[e], slice_base);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     float a[3], b[3];
-    load_node<kStorage>(c.e[j >> 1], j & 1, a[0], a[1], a[2]);
-    load_node<kStorage>(c.e[2 + (j >> 1)], j & 1, b[0], b[1], b[2]);
+    load_node<kStorage>(at[j >> 1], j & 1, a[0], a[1], a[2]);
+    load_node<kStorage>(at[2 + (j >> 1)], j & 1, b[0], b[1], b[2]);
 #pragma unroll
     for (int i = 0; i < 3; ++i) k.p[j][i] = make_float2(a[i], b[i]);
   }
 }
 
 template <int kStorage>
-__device__ __forceinline__ void gather(const FieldView& f, uint32_t node, CornerEdges& k,
+__device__ __forceinline__ void gather(const FieldView& f, const CellRows& rows, CornerEdges& k,
                                        int64_t slice_base = 0) {
-  const char* base = static_cast<const char*>(f.nodes) +
-                     (uint64_t(slice_base) + node) * uint64_t(kEdgeRecordBytes);
-  const uint64_t s1 = uint64_t(f.stride1) * kEdgeRecordBytes;
-  const uint64_t s0 = uint64_t(f.stride0) * kEdgeRecordBytes;
-  load_edge_record(base, k.z[0]);
-  load_edge_record(base + s1, k.z[1]);
-  load_edge_record(base + s0, k.z[2]);
-  load_edge_record(base + s0 + s1, k.z[3]);
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    load_edge_record(static_cast<const char*>(f.nodes) +
+                         (uint64_t(slice_base) + rows.at[e]) * uint64_t(kEdgeRecordBytes),
+                     k.z[e]);
 }
 
 __device__ __forceinline__ void trilinear(const FieldView& f, const CornerNodes& k,
@@ -381,9 +396,12 @@ __device__ __forceinline__ void trilinear(const FieldView&, const CornerEdges& k
 
 // A per-thread cache of the current cell's corners: a particle usually stays
 // in one cell for several steps, and the sampled values do not depend on
-// whether the corners came from the cache or from memory.
-template <int kStorage, int kLocate>
+// whether the corners came from the cache or from memory. kMode is the field's
+// LocateMode, with kTiledBit for a tiled field.
+template <int kStorage, int kMode>
 struct CellSampler {
+  static constexpr int kLocate = kMode & ~kTiledBit;
+  static constexpr bool kTiled = (kMode & kTiledBit) != 0;
   CornersOf<kStorage> corners;
   uint32_t cached = ~0u;  // first node of the cached cell (no cell starts there)
 
@@ -395,10 +413,10 @@ struct CellSampler {
     Cell c;
     Weights w;
     if (!locate<kLocate>(f, p, c, w)) return false;
-    const uint32_t node = first_node(f, c);
-    if (node != cached) {
-      gather<kStorage>(f, node, corners);
-      cached = node;
+    const CellRows rows = cell_rows<kTiled>(f, c);
+    if (rows.at[0] != cached) {
+      gather<kStorage>(f, rows, corners);
+      cached = rows.at[0];
     }
     trilinear(f, corners, w, v01, v2);
     return true;
@@ -412,14 +430,14 @@ struct CellSampler {
     Cell c;
     Weights w;
     const bool inside = locate<kLocate>(f, p, c, w);
-    const uint32_t node = first_node(f, c);
-    const bool need = inside && node != cached;
+    const CellRows rows = cell_rows<kTiled>(f, c);
+    const bool need = inside && rows.at[0] != cached;
     if constexpr (kStorage == DPA_STORAGE_F32) {
-      gather_if(f, node, need, corners);
-      cached = need ? node : cached;
+      gather_if(f, rows, need, corners);
+      cached = need ? rows.at[0] : cached;
     } else if (need) {
-      gather<kStorage>(f, node, corners);
-      cached = node;
+      gather<kStorage>(f, rows, corners);
+      cached = rows.at[0];
     }
     trilinear(f, corners, w, v01, v2);
     return inside;
@@ -469,14 +487,14 @@ struct TimeSampler {
     Cell c;
     Weights w;
     if (!locate<kLocate>(f, p, c, w)) return false;
-    const uint32_t node = first_node(f, c);
+    const CellRows rows = cell_rows<false>(f, c);
     int64_t slice = 0;
     float wt = 0.0f;
     if (!locate_time(f, t, slice, wt)) return false;
-    if (node != cached || slice != cached_slice) {
-      gather<kStorage>(f, node, lo, slice);
-      gather<kStorage>(f, node, hi, slice + f.slice_stride);
-      cached = node;
+    if (rows.at[0] != cached || slice != cached_slice) {
+      gather<kStorage>(f, rows, lo, slice);
+      gather<kStorage>(f, rows, hi, slice + f.slice_stride);
+      cached = rows.at[0];
       cached_slice = slice;
     }
     float2 a01, b01;
