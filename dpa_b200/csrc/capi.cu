@@ -669,7 +669,9 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     v.time_spacing = slices > 1 ? time_spacing : 1.0f;
     split_reciprocal(v.time_spacing, &v.time_reciprocal, &v.time_reciprocal_lo);
     v.time_fast = 0;
-    if (slices > 1 && !ctx->ieee_division) {
+    // The ranges that locate_time()'s single test rests on.
+    if (slices > 1 && !ctx->ieee_division && slices <= (1u << 23) &&
+        v.time_spacing >= std::ldexp(1.0f, -40) && v.time_spacing <= std::ldexp(1.0f, 40)) {
       bool exact = false;
       const int st = reciprocal_divides_exactly(ctx, v.time_spacing, &exact);
       if (st != DPA_OK) {
@@ -680,6 +682,7 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
       v.time_fast = exact ? 1 : 0;
     }
     v.time_upper = float(int64_t(slices) - 1);
+    v.time_cells = slices - 1;
     *out = f;
     return DPA_OK;
   });

@@ -85,7 +85,8 @@ struct FieldView {
   float time_reciprocal;     // RN(1 / time_spacing)
   float time_reciprocal_lo;  // RN(1 / time_spacing - time_reciprocal)
   int32_t time_fast;         // the time axis divides as kLocateReciprocal
-  float time_upper;      // slices - 1: inside iff 0 <= (t - t0) / dt < slices - 1
+  float time_upper;          // slices - 1: inside iff 0 <= (t - t0) / dt < slices - 1
+  uint32_t time_cells;       // the same as an integer
 };
 
 // a / h by a known divisor: with y + yl = 1 / h split into two floats,

@@ -451,22 +451,27 @@ struct CellSampler {
 };
 
 // The time axis of a time-varying field, located by the spatial rule: slice
-// s = floor((t - t0) / dt) of the rounded quotient, weight fmod(t - t0, dt) / dt,
-// inside iff 0 <= s <= slices - 2. Returns the first node of slice s.
-__device__ __forceinline__ bool locate_time(const FieldView& f, float t, int64_t& slice_base,
-                                            float& w) {
+// k = floor((t - t0) / dt) of the rounded quotient, weight fmod(t - t0, dt) / dt,
+// inside iff 0 <= k <= slices - 2. time_fast fields (spacing in [2^-40, 2^40], at
+// most 2^23 slices) divide and take the floor as locate() does, without the
+// conversions and the branches of the guarded divisions.
+__device__ __forceinline__ bool locate_time(const FieldView& f, float t, uint32_t& k, float& w) {
   const float a = __fsub_rn(t, f.time_origin);
-  const float y = f.time_reciprocal, yl = f.time_reciprocal_lo;
-  const float q = f.time_fast ? divide_by_reciprocal(a, f.time_spacing, y, yl)
-                              : __fdiv_rn(a, f.time_spacing);
+  const float y = f.time_reciprocal, yl = f.time_reciprocal_lo, h = f.time_spacing;
+  if (f.time_fast && a >= 0x1p-64f) {
+    const float b = __fadd_rd(__fmaf_rn(a, y, __fmul_rn(a, yl)), 0x1p23f);
+    k = __float_as_uint(b) - 0x4B000000u;
+    float r = __fmaf_rn(-__fsub_rn(b, 0x1p23f), h, a);
+    if (r < 0.0f) r = __fadd_rn(r, h);
+    w = __fmaf_rn(r, y, __fmul_rn(r, yl));
+    return k < f.time_cells;
+  }
+  const float q = f.time_fast ? divide_by_reciprocal(a, h, y, yl) : __fdiv_rn(a, h);
   if (!(q >= 0.0f && q < f.time_upper)) return false;
   const float s = floorf(q);
-  float r = fmaf(-s, f.time_spacing, a);
-  if (r < 0.0f) r = __fadd_rn(r, f.time_spacing);
-  if (r == 0.0f) r = copysignf(0.0f, a);
-  w = f.time_fast ? divide_by_reciprocal(r, f.time_spacing, y, yl)
-                   : __fdiv_rn(r, f.time_spacing);
-  slice_base = int64_t(uint64_t(uint32_t(s)) * uint64_t(f.slice_stride));
+  const float r = remainder_general(a, s, h);
+  w = f.time_fast ? divide_by_reciprocal(r, h, y, yl) : __fdiv_rn(r, h);
+  k = uint32_t(s);
   return true;
 }
 
@@ -479,8 +484,7 @@ __device__ __forceinline__ bool locate_time(const FieldView& f, float t, int64_t
 template <int kStorage, int kLocate>
 struct TimeSampler {
   CornersOf<kStorage> lo, hi;  // slices s and s + 1
-  uint32_t cached = ~0u;
-  int64_t cached_slice = -1;
+  uint32_t cached = ~0u, cached_slice = 0;
 
   __device__ __forceinline__ bool sample(const FieldView& f, const Position& p, float t,
                                          float2& v01, float& v2) {
@@ -488,12 +492,13 @@ struct TimeSampler {
     Weights w;
     if (!locate<kLocate>(f, p, c, w)) return false;
     const CellRows rows = cell_rows<false>(f, c);
-    int64_t slice = 0;
+    uint32_t slice = 0;
     float wt = 0.0f;
     if (!locate_time(f, t, slice, wt)) return false;
     if (rows.at[0] != cached || slice != cached_slice) {
-      gather<kStorage>(f, rows, lo, slice);
-      gather<kStorage>(f, rows, hi, slice + f.slice_stride);
+      const int64_t base = int64_t(uint64_t(slice) * uint32_t(f.slice_stride));
+      gather<kStorage>(f, rows, lo, base);
+      gather<kStorage>(f, rows, hi, base + f.slice_stride);
       cached = rows.at[0];
       cached_slice = slice;
     }
@@ -510,10 +515,7 @@ struct TimeSampler {
   static constexpr bool kSteady = false;
   static constexpr bool kPackedSums = true;
 
-  __device__ __forceinline__ void reset() {
-    cached = ~0u;
-    cached_slice = -1;
-  }
+  __device__ __forceinline__ void reset() { cached = ~0u; }
 };
 
 __device__ __forceinline__ bool is_zero(float2 v01, float v2) {

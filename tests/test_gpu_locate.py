@@ -37,3 +37,28 @@ def test_starts_on_faces_and_cell_boundaries(ctx, oracle, spacing, storage):
     assert_same(got.termination, want.termination)
     assert_same(got.remaining_iterations, want.remaining)
     assert_same(got.position, want.positions)
+
+
+@pytest.mark.parametrize("spacing", [0.7, 1.0 / 3.0, 3e-13, 3e12])
+def test_starts_on_slice_boundaries(ctx, oracle, spacing):
+    """The time axis likewise: starts at the first slice, before it, on and
+    beside later ones and past the last."""
+    rng = np.random.default_rng(6)
+    data = rng.integers(-8, 9, (5, 4, 6, 5, 3)).astype(np.float32)
+    dt = np.float32(spacing)
+    grid = dpa_b200.UnsteadyGrid.from_data(data, (0.7, 0.7, 0.7), dt)
+    slices = (dt * np.arange(6, dtype=np.float32)).astype(np.float32)
+    values = np.concatenate([np.float32([0.0, -0.0, 2.0 ** -64, 1e-30, -1e-30]), slices,
+                             np.nextafter(slices, np.float32(-1)),
+                             np.nextafter(slices, np.float32(np.inf)), dt * np.float32([0.4, 2.6])])
+    pos = (rng.random((3000, 3)) * [2.1, 3.5, 2.8]).astype(np.float32)
+    t0 = values[rng.integers(0, len(values), 3000)].astype(np.float32)
+    step, rem = float(np.float32(0.01) * dt), np.full(3000, 30, np.uint64)
+    field = ctx.field(grid)
+    for integrator in ("runge_kutta_4", "runge_kutta_4_true"):
+        want = oracle.advect_pathlines(grid, integrator, step, pos, t0, rem)
+        got = dpa_b200.advect_pathlines(ctx, field, pos, t0, 30, integrator, step)
+        assert_same(got.termination, want.termination)
+        assert_same(got.position, want.positions)
+        assert_same(got.time, want.times)
+    field.close()
