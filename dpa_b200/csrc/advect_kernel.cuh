@@ -45,7 +45,9 @@ constexpr int advect_min_blocks() {
 // Persistent advection. Every lane owns kPPT slots, each holding one particle
 // at a time; a slot whose particle finishes takes the next one from its
 // warp's claim of a.claim consecutive entries of the processing order, and
-// the warp claims a new batch with one atomic when its batch runs out. Lanes
+// the warp claims a new batch with one atomic when its batch runs out. A launch
+// with a slot for every particle needs no claims: each warp is given its own
+// entries (work_counter null). Lanes
 // therefore stay busy while particles of one warp end after very different
 // numbers of steps. A particle takes at most a.max_steps steps per launch;
 // one stopped by that budget alone is reported as in flight and resumes in a
@@ -79,7 +81,12 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
   const unsigned tid = threadIdx.x;
   const unsigned lane = tid & 31u;
   uint64_t* const warp_claim = claims[tid >> 5];
-  if (lane == 0) warp_claim[0] = warp_claim[1] = 0;
+  if (lane == 0) {
+    const uint64_t size = a.work_counter ? 0 : 32u * kPPT;
+    const uint64_t own = (uint64_t(blockIdx.x) * (blockDim.x >> 5) + (tid >> 5)) * size;
+    warp_claim[0] = own < a.count ? own : a.count;
+    warp_claim[1] = own + size < a.count ? own + size : a.count;
+  }
   __syncwarp();
   bool exhausted = false;
   // Where an empty slot waits: the centre of the first cell, so that a step
@@ -118,8 +125,9 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
       while (idle && !exhausted) {
         uint64_t next = warp_claim[0], end = warp_claim[1];
         if (next == end) {
-          unsigned long long base = 0;
-          if (lane == 0) base = atomicAdd(a.work_counter, (unsigned long long)claim);
+          unsigned long long base = a.count;
+          if (lane == 0 && a.work_counter)
+            base = atomicAdd(a.work_counter, (unsigned long long)claim);
           base = __shfl_sync(kFull, base, 0);
           if (base >= a.count) {
             exhausted = true;
@@ -349,9 +357,13 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
   const uint64_t needed = (lanes + block - 1) / block;
   const uint64_t blocks = std::min<uint64_t>(needed, uint64_t(resident) * uint64_t(sms));
   if (blocks == 0) return cudaSuccess;
-  DPA_CUDA_TRY(cudaMemsetAsync(a.work_counter, 0, sizeof(unsigned long long), stream));
+  AdvectArgs launch = a;
+  if (blocks == needed)
+    launch.work_counter = nullptr;
+  else
+    DPA_CUDA_TRY(cudaMemsetAsync(a.work_counter, 0, sizeof(unsigned long long), stream));
   advect_kernel<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>
-      <<<dim3(unsigned(blocks)), dim3(block), 0, stream>>>(f, a);
+      <<<dim3(unsigned(blocks)), dim3(block), 0, stream>>>(f, launch);
   return cudaGetLastError();
 }
 

@@ -138,6 +138,9 @@ int advect_device_impl(dpa_context* ctx, const dpa_field* field, const dpa_advec
   return DPA_OK;
 }
 
+// Raw curves up to which a piece is emitted before its totals are known.
+constexpr uint64_t kEarlyEmitBytes = 64ull << 20;
+
 // Advects and emits particles [begin, end) of a recording round. The device
 // arrays ctx->positions / remaining hold the whole round.
 int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_options* o,
@@ -147,16 +150,16 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
   cudaStream_t s = ctx->stream;
   const uint64_t n = end - begin;
   // Raw (unpruned) vertex offsets: remaining + 2 slots per particle.
-  DPA_TRY_CUDA(ctx, ctx->host_offsets.reserve(n * 8));
+  DPA_TRY_CUDA(ctx, ctx->host_offsets.reserve((n + 1) * 8));
   uint64_t* offsets = ctx->host_offsets.as<uint64_t>();
   uint64_t raw_total = 0;
   for (uint64_t i = 0; i < n; ++i) {
     offsets[i] = raw_total;
     raw_total += host_remaining[begin + i] + 2;
   }
+  offsets[n] = raw_total;
   DPA_TRY_CUDA(ctx, ctx->raw.reserve(raw_total * 12));
-  DPA_TRY_CUDA(ctx, ctx->raw_offsets.reserve(n * 8));
-  DPA_TRY_CUDA(ctx, ctx->raw_counts.reserve(n * 8));
+  DPA_TRY_CUDA(ctx, ctx->raw_offsets.reserve((n + 1) * 8));
   DPA_TRY_CUDA(ctx, ctx->kept_vertices.reserve(n * 4));
   DPA_TRY_CUDA(ctx, ctx->kept_segments.reserve(n * 4));
   DPA_TRY_CUDA(ctx, ctx->vertex_offsets.reserve(n * 8));
@@ -165,8 +168,8 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
   DPA_TRY_CUDA(ctx, ctx->host_totals.reserve(32));
   // The pinned offsets of the previous piece are free: its copies finished
   // before the previous piece returned.
-  DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->raw_offsets.ptr, offsets, n * 8, cudaMemcpyHostToDevice,
-                                    s));
+  DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->raw_offsets.ptr, offsets, (n + 1) * 8,
+                                    cudaMemcpyHostToDevice, s));
 
   float* positions = ctx->positions.as<float>() + 3 * begin;
   uint64_t* remaining = ctx->remaining.as<uint64_t>() + begin;
@@ -200,38 +203,30 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
     DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[3], s));
   }
 
-  // Per-particle raw counts, then piece-local offsets of kept vertices and
-  // kept segments and their totals.
-  DPA_TRY_CUDA(ctx, dpa::launch_raw_counts(ctx->remaining_in.as<uint64_t>() + begin, remaining, n,
-                                           ctx->raw_counts.as<uint64_t>(), s));
+  // Piece-local offsets of kept vertices and kept segments and their totals.
   DPA_TRY_CUDA(ctx, ctx->scan_temp.reserve(dpa::curve_offsets_scratch_bytes(n)));
   DPA_TRY_CUDA(ctx, dpa::launch_curve_offsets(
                         ctx->kept_vertices.as<uint32_t>(), ctx->kept_segments.as<uint32_t>(), n,
                         ctx->scan_temp.ptr, ctx->vertex_offsets.as<uint64_t>(),
                         ctx->segment_offsets.as<uint64_t>(),
                         ctx->totals.as<unsigned long long>(), s));
-  ctx->launches += 1 + dpa::kCurveOffsetsLaunches;
+  ctx->launches += uint64_t(dpa::curve_offsets_launches(n));
   uint64_t* ht = ctx->host_totals.as<uint64_t>();
   DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ht, ctx->totals.ptr, 16, cudaMemcpyDeviceToHost, s));
-  DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
-  const uint64_t piece_vertices = ht[0];
-  const uint64_t piece_segments = ht[1];
-  const uint64_t piece_indices = 2 * piece_segments;
-  if (!o->index64 && *round_vertices + piece_vertices > 0xffffffffull)
-    return fail(ctx, DPA_ERROR_UNSUPPORTED,
-                "the round's curve has more vertices than 32-bit indices can address; "
-                "set index64");
-
   const size_t index_bytes = o->index64 ? 8 : 4;
-  DPA_TRY_CUDA(ctx, ctx->out_vertices.reserve(piece_vertices * 12));
-  DPA_TRY_CUDA(ctx, ctx->out_colors.reserve(piece_vertices * 4));
-  DPA_TRY_CUDA(ctx, ctx->out_indices.reserve(piece_indices * index_bytes));
+  // A small piece is emitted without waiting for its totals, into room for all
+  // of its raw vertices; a large one waits, and takes no more than it needs.
+  const bool early = raw_total * 12 <= kEarlyEmitBytes;
+  if (!early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+  DPA_TRY_CUDA(ctx, ctx->out_vertices.reserve((early ? raw_total : ht[0]) * 12));
+  DPA_TRY_CUDA(ctx, ctx->out_colors.reserve((early ? raw_total : ht[0]) * 4));
+  DPA_TRY_CUDA(ctx, ctx->out_indices.reserve(2 * (early ? raw_total : ht[1]) * index_bytes));
 
   dpa::EmitArgs e{};
   e.count = n;
   e.raw_vertices = ctx->raw.as<float>();
   e.raw_offsets = ctx->raw_offsets.as<uint64_t>();
-  e.steps_raw = ctx->raw_counts.as<uint64_t>();
+  e.remaining = remaining;
   e.vertex_offsets = ctx->vertex_offsets.as<uint64_t>();
   e.segment_offsets = ctx->segment_offsets.as<uint64_t>();
   e.kept_vertices = ctx->kept_vertices.as<uint32_t>();
@@ -242,6 +237,14 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
   DPA_TRY_CUDA(ctx, dpa::launch_emit(e, o->index64 != 0, o->colors != 0, s));
   ctx->launches += 1;
   if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[4], s));
+  if (early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+  const uint64_t piece_vertices = ht[0];
+  const uint64_t piece_segments = ht[1];
+  const uint64_t piece_indices = 2 * piece_segments;
+  if (!o->index64 && *round_vertices + piece_vertices > 0xffffffffull)
+    return fail(ctx, DPA_ERROR_UNSUPPORTED,
+                "the round's curve has more vertices than 32-bit indices can address; "
+                "set index64");
 
   // The piece's curve crosses to the host in chunks through two pinned
   // halves, so that chunk j + 1 copies while the sink takes chunk j and the
@@ -797,9 +800,6 @@ int dpa_advect_round(dpa_context* ctx, const dpa_field* field, const dpa_advect_
                               ctx->remaining.as<uint64_t>(), ctx->termination.as<uint8_t>(), s);
       if (st != DPA_OK) return st;
     } else {
-      DPA_TRY_CUDA(ctx, ctx->remaining_in.reserve(count * 8));
-      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->remaining_in.ptr, ctx->remaining.ptr, count * 8,
-                                        cudaMemcpyDeviceToDevice, s));
       ctx->round_order_ms = ctx->round_advect_ms = ctx->round_emit_ms = 0.0f;
       // Pieces of the round whose unpruned curves fit the staging limit.
       const uint64_t limit_vertices = std::max<uint64_t>(ctx->staging_limit / 12, 1);

@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(kEmitWarps * 32) emit_kernel(const EmitArgs e)
 
   // Pass 1: copy the particle's surviving raw vertices to their pruned slots.
   const float* raw = e.raw_vertices + 3 * e.raw_offsets[k];
-  const uint64_t raw_count = e.steps_raw[k];
+  const uint64_t raw_in = e.remaining_in ? e.remaining_in[k] + 2 : e.raw_offsets[k + 1] - e.raw_offsets[k];
+  const uint64_t raw_count = raw_in - e.remaining[k];
   const uint64_t first = e.vertex_offsets[k];
   uint64_t cursor = first;
   for (uint64_t j0 = 0; j0 < raw_count; j0 += 32) {
@@ -139,12 +140,6 @@ __global__ void __launch_bounds__(kEmitWarps * 32) emit_kernel(const EmitArgs e)
       }
     }
   }
-}
-
-__global__ void raw_counts_kernel(const uint64_t* in, const uint64_t* out, uint64_t count,
-                                  uint64_t* raw) {
-  const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t < count) raw[t] = in[t] - out[t] + 2;
 }
 
 // Curve offsets: the exclusive scans of the per-particle kept-vertex and
@@ -260,6 +255,32 @@ __global__ void __launch_bounds__(kScanThreads) offsets_tiles_kernel(
   }
 }
 
+// The three passes as one block's, for few particles: launches cost more there
+// than the scan (4096 particles: three kernels and their gaps 9 us, this 5).
+constexpr int kOneBlockThreads = 1024;
+__global__ void __launch_bounds__(kOneBlockThreads) offsets_one_block_kernel(
+    const uint32_t* a, const uint32_t* b, uint64_t n, uint64_t* out_a, uint64_t* out_b,
+    unsigned long long* totals) {
+  __shared__ ulonglong2 warp_sums[kOneBlockThreads / 32];
+  ulonglong2 carry = make_ulonglong2(0, 0);
+  for (uint64_t base = 0; base < n; base += kOneBlockThreads) {
+    const uint64_t i = base + threadIdx.x;
+    const ulonglong2 v = load_counts(a, b, n, i);
+    ulonglong2 total;
+    const ulonglong2 ex = block_exclusive_scan2(v, warp_sums, &total);
+    if (i < n) {
+      out_a[i] = carry.x + ex.x;
+      out_b[i] = carry.y + ex.y;
+    }
+    carry.x += total.x;
+    carry.y += total.y;
+  }
+  if (threadIdx.x == 0) {
+    totals[0] = carry.x;
+    totals[1] = carry.y;
+  }
+}
+
 // Node layouts: one float4 (F32) or (x, y, z, 0) half/bfloat quad per node.
 // F32_EDGES: record t holds nodes t and t + 1 along axis 2, each component's
 // pair side by side (sample.cuh); the last node of a row repeats itself, and
@@ -330,14 +351,6 @@ cudaError_t launch_emit(const EmitArgs& e, bool index64, bool colors, cudaStream
   return cudaGetLastError();
 }
 
-cudaError_t launch_raw_counts(const uint64_t* remaining_in, const uint64_t* remaining_out,
-                              uint64_t count, uint64_t* raw_counts, cudaStream_t stream) {
-  if (count == 0) return cudaSuccess;
-  raw_counts_kernel<<<blocks_for(count, 256), 256, 0, stream>>>(remaining_in, remaining_out, count,
-                                                                raw_counts);
-  return cudaGetLastError();
-}
-
 uint64_t curve_offsets_scratch_bytes(uint64_t count) {
   return ((count + kScanTileItems - 1) / kScanTileItems) * sizeof(ulonglong2) + 16;
 }
@@ -347,6 +360,11 @@ cudaError_t launch_curve_offsets(const uint32_t* kept_vertices, const uint32_t* 
                                  uint64_t* segment_offsets, unsigned long long* totals,
                                  cudaStream_t stream) {
   if (count == 0) return cudaMemsetAsync(totals, 0, 16, stream);
+  if (count <= kOneBlockOffsets) {
+    offsets_one_block_kernel<<<1, kOneBlockThreads, 0, stream>>>(
+        kept_vertices, kept_segments, count, vertex_offsets, segment_offsets, totals);
+    return cudaGetLastError();
+  }
   const uint64_t tiles = (count + kScanTileItems - 1) / kScanTileItems;
   if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
   ulonglong2* sums = static_cast<ulonglong2*>(scratch);

@@ -126,7 +126,7 @@ struct dpa_context {
   bool timed_round = false;
   float round_order_ms = 0.0f, round_advect_ms = 0.0f, round_emit_ms = 0.0f;
   dpa_tuning_state tuning;
-  DeviceBuffer raw, raw_offsets, raw_counts, kept_vertices, kept_segments;
+  DeviceBuffer raw, raw_offsets, kept_vertices, kept_segments;
   DeviceBuffer wide, vertex_offsets, segment_offsets, scan_temp, totals;
   DeviceBuffer out_vertices, out_colors, out_indices;
   PinnedBuffer host_vertices, host_colors, host_indices, host_totals, host_offsets;
@@ -135,7 +135,6 @@ struct dpa_context {
   void release_all() {
     scratch.release();
     DeviceBuffer* d[] = {&positions, &remaining, &remaining_in, &termination, &raw, &raw_offsets,
-                         &raw_counts,
                          &kept_vertices, &kept_segments, &wide, &vertex_offsets,
                          &segment_offsets, &scan_temp, &totals, &out_vertices, &out_colors,
                          &out_indices, &ftle_winners, &ftle_out, &ftle_original,

@@ -58,7 +58,8 @@ struct AdvectArgs {
                                      // kAdvectBlock; 0 = kAdvectBlock, or fewer when
                                      // the particles would not reach every SM
   uint32_t particles_per_thread;     // 1 or 2 (2: steady fields without recording)
-  unsigned long long* work_counter;  // zeroed by the launcher; claims of the order
+  unsigned long long* work_counter;  // claims of the order; the launcher zeroes it, or
+                                     // passes null when every particle has a slot
   // Recording only.
   float* raw_vertices;          // unpruned curve of particle k at raw_offsets[k]
   const uint64_t* raw_offsets;  // exclusive scan of remaining + 2
@@ -140,7 +141,10 @@ struct EmitArgs {
   uint64_t count;                 // particles in this piece, in round order
   const float* raw_vertices;
   const uint64_t* raw_offsets;    // per particle
-  const uint64_t* steps_raw;      // per particle: raw vertex count (steps + 2)
+  const uint64_t* remaining;      // per particle, after its last step
+  const uint64_t* remaining_in;   // before its first; null: the raw curves lie one after
+                                  // another, remaining_in + 2 vertices each, and
+                                  // raw_offsets holds count + 1 entries
   const uint64_t* vertex_offsets; // exclusive scan of kept vertices (piece-local)
   const uint64_t* segment_offsets;// exclusive scan of kept segments (piece-local)
   const uint32_t* kept_vertices;
@@ -152,20 +156,17 @@ struct EmitArgs {
 
 cudaError_t launch_emit(const EmitArgs& e, bool index64, bool colors, cudaStream_t stream);
 
-// Raw vertex count per particle: remaining_in - remaining_out + 2.
-cudaError_t launch_raw_counts(const uint64_t* remaining_in, const uint64_t* remaining_out,
-                              uint64_t count, uint64_t* raw_counts, cudaStream_t stream);
-
 // Exclusive scans of the per-particle kept-vertex and kept-segment counts
-// into vertex_offsets and segment_offsets (three kernels); totals (device,
-// two entries) receives the sums of both. scratch holds
+// into vertex_offsets and segment_offsets (one kernel up to kOneBlockOffsets
+// particles, three beyond); totals (device, two entries) receives the sums of both. scratch holds
 // curve_offsets_scratch_bytes(count) bytes.
 uint64_t curve_offsets_scratch_bytes(uint64_t count);
 cudaError_t launch_curve_offsets(const uint32_t* kept_vertices, const uint32_t* kept_segments,
                                  uint64_t count, void* scratch, uint64_t* vertex_offsets,
                                  uint64_t* segment_offsets, unsigned long long* totals,
                                  cudaStream_t stream);
-constexpr int kCurveOffsetsLaunches = 3;
+constexpr uint64_t kOneBlockOffsets = 8192;
+inline int curve_offsets_launches(uint64_t count) { return count <= kOneBlockOffsets ? 1 : 3; }
 
 // The data-path probe of dpa_measure_gather_bandwidth: blocks x 256 lanes,
 // each loading 8 16-byte nodes per iteration from table (mask + 1 nodes).

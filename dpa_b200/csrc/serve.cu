@@ -100,7 +100,7 @@ struct dpa_server {
   cudaEvent_t seeds_copied = nullptr, readback[2] = {nullptr, nullptr};
   cudaEvent_t tick_start[2] = {nullptr, nullptr};  // device time of each tick
   // Emission scratch.
-  DeviceBuffer raw_counts, curve_totals, vertex_offsets, segment_offsets, scan_temp, out_vertices,
+  DeviceBuffer curve_totals, vertex_offsets, segment_offsets, scan_temp, out_vertices,
       out_colors, out_indices;
   DeviceBuffer ftle_original, ftle_winners, ftle_out;
   range_allocator slots, vertices;
@@ -447,12 +447,8 @@ void dpa_server::finish(active_request& a, response_storage& out) {
   if (record) {
     // Emission of the request's curve, as one round of the reference:
     // offsets and totals first, to size the response.
-    SERVER_TRY(raw_counts.reserve(n * 8));
     SERVER_TRY(vertex_offsets.reserve(n * 8));
     SERVER_TRY(segment_offsets.reserve(n * 8));
-    SERVER_TRY(dpa::launch_raw_counts(remaining_initial.as<uint64_t>() + first,
-                                      remaining.as<uint64_t>() + first, n,
-                                      raw_counts.as<uint64_t>(), finish_stream));
     SERVER_TRY(scan_temp.reserve(dpa::curve_offsets_scratch_bytes(n)));
     SERVER_TRY(curve_totals.reserve(16));
     SERVER_TRY(dpa::launch_curve_offsets(kept_vertices.as<uint32_t>() + first,
@@ -529,7 +525,8 @@ void dpa_server::finish(active_request& a, response_storage& out) {
     e.count = n;
     e.raw_vertices = raw.as<float>();
     e.raw_offsets = raw_offsets.as<uint64_t>() + first;
-    e.steps_raw = raw_counts.as<uint64_t>();
+    e.remaining = remaining.as<uint64_t>() + first;
+    e.remaining_in = remaining_initial.as<uint64_t>() + first;
     e.vertex_offsets = vertex_offsets.as<uint64_t>();
     e.segment_offsets = segment_offsets.as<uint64_t>();
     e.kept_vertices = kept_vertices.as<uint32_t>() + first;
