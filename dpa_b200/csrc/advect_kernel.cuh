@@ -47,7 +47,7 @@ constexpr int advect_min_blocks() {
 // warp's claim of a.claim consecutive entries of the processing order, and
 // the warp claims a new batch with one atomic when its batch runs out. A launch
 // with a slot for every particle needs no claims: each warp is given its own
-// entries (work_counter null). Lanes
+// a.own_entries entries (work_counter null). Lanes
 // therefore stay busy while particles of one warp end after very different
 // numbers of steps. A particle takes at most a.max_steps steps per launch;
 // one stopped by that budget alone is reported as in flight and resumes in a
@@ -82,7 +82,7 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
   const unsigned lane = tid & 31u;
   uint64_t* const warp_claim = claims[tid >> 5];
   if (lane == 0) {
-    const uint64_t size = a.work_counter ? 0 : 32u * kPPT;
+    const uint64_t size = a.work_counter ? 0 : a.own_entries;
     const uint64_t own = (uint64_t(blockIdx.x) * (blockDim.x >> 5) + (tid >> 5)) * size;
     warp_claim[0] = own < a.count ? own : a.count;
     warp_claim[1] = own + size < a.count ? own + size : a.count;
@@ -338,6 +338,19 @@ inline uint32_t advect_block(const AdvectArgs& a, uint64_t lanes, int sms) {
   return block;
 }
 
+// Particles per warp of a small launch: as few as keep every SM at 8 warps or
+// less (1, 2, 4, 8, 16; else 32). A warp waits at every step for the slowest of its
+// lanes' gathers, and such a launch leaves the SMs' issue slots idle; more warps per
+// SM than that take turns instead. B200, us at 32 lanes and as chosen: 100 recorded
+// seeds 33 -> 21 (1 lane), 1000 216 -> 168 (1), 4096 245 -> 200 (4), 16,384 202 ->
+// 178 (16); end positions of 8000 seeds in a 256^3 field 227 -> 191 (8), in F16 fields
+// that L2 holds 119 -> 121; pathlines of 8000 seeds 262 -> 214.
+inline uint32_t particles_per_warp(uint64_t count, int sms) {
+  uint32_t lanes = 1;
+  while (lanes < 32 && count > uint64_t(lanes) * 8u * uint64_t(sms)) lanes *= 2;
+  return lanes;
+}
+
 template <int kIntegrator, int kStorage, int kLocate, bool kRecord, bool kUnsteady, int kPPT>
 cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t stream) {
   // Persistent grid: as many blocks as fit on the device at once (or as the
@@ -346,7 +359,9 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
   int sms = 0, resident = 0;
   DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>(
       kAdvectBlock, &resident, &sms)));
-  const uint32_t block = advect_block(a, lanes, sms);
+  const bool free_shape = kPPT == 1 && !a.block && !a.blocks_per_sm;
+  const uint32_t own = free_shape ? particles_per_warp(a.count, sms) : 32u * kPPT;
+  const uint32_t block = own < 32 ? 32 : advect_block(a, lanes, sms);
   if (block == 0 || block % 32 != 0 || block > uint32_t(kAdvectBlock)) return cudaErrorInvalidValue;
   DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>(
       block, &resident, &sms)));
@@ -354,10 +369,12 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
   if (a.blocks_per_sm && int(a.blocks_per_sm) < resident) resident = int(a.blocks_per_sm);
   if (!a.blocks_per_sm && f.threads_per_sm)
     resident = std::min(resident, std::max(1, int(f.threads_per_sm / block)));
-  const uint64_t needed = (lanes + block - 1) / block;
+  const uint64_t per_block = uint64_t(block / 32) * own;
+  const uint64_t needed = (a.count + per_block - 1) / per_block;
   const uint64_t blocks = std::min<uint64_t>(needed, uint64_t(resident) * uint64_t(sms));
   if (blocks == 0) return cudaSuccess;
   AdvectArgs launch = a;
+  launch.own_entries = own;
   if (blocks == needed)
     launch.work_counter = nullptr;
   else

@@ -60,6 +60,7 @@ struct AdvectArgs {
   uint32_t particles_per_thread;     // 1 or 2 (2: steady fields without recording)
   unsigned long long* work_counter;  // claims of the order; the launcher zeroes it, or
                                      // passes null when every particle has a slot
+  uint32_t own_entries;              // then each warp's entries; set by the launcher
   // Recording only.
   float* raw_vertices;          // unpruned curve of particle k at raw_offsets[k]
   const uint64_t* raw_offsets;  // exclusive scan of remaining + 2
