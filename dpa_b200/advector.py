@@ -328,12 +328,9 @@ class ParticleAdvector:
             # compute_round_state (particle_advector.cpp:261-310): the tail.
             count = min(self.particles_per_round, active)
             lo, hi = active - count, active
-            pos = np.ascontiguousarray(positions[lo:hi])
-            rem = np.ascontiguousarray(remaining[lo:hi])
-            term, curve = self.advect_round(field, pos, rem, index64)
-            positions[lo:hi] = pos
-            remaining[lo:hi] = rem
-            termination[lo:hi] = term
+            # Slices of contiguous arrays: updated in place.
+            termination[lo:hi], curve = self.advect_round(field, positions[lo:hi],
+                                                          remaining[lo:hi], index64)
             if curve is not None:
                 curves.append(curve)
             active = lo

@@ -141,43 +141,52 @@ int advect_device_impl(dpa_context* ctx, const dpa_field* field, const dpa_advec
 // Raw curves up to which a piece is emitted before its totals are known.
 constexpr uint64_t kEarlyEmitBytes = 64ull << 20;
 
-// Advects and emits particles [begin, end) of a recording round. The device
-// arrays ctx->positions / remaining hold the whole round.
-int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_options* o,
-                 const dpa::StepCoefficients& k, uint64_t begin, uint64_t end,
-                 const uint64_t* host_remaining, uint64_t* round_vertices,
-                 uint64_t* round_indices, bool final_piece, dpa_curve_sink sink, void* user) {
-  cudaStream_t s = ctx->stream;
-  const uint64_t n = end - begin;
-  // Raw (unpruned) vertex offsets: remaining + 2 slots per particle.
-  DPA_TRY_CUDA(ctx, ctx->host_offsets.reserve((n + 1) * 8));
-  uint64_t* offsets = ctx->host_offsets.as<uint64_t>();
-  uint64_t raw_total = 0;
+// Rounds of up to this many particles pass through pinned memory, one copy each
+// way; the driver stages each of the arrays of a larger one itself, or takes them
+// from pinned memory of the caller's.
+constexpr uint64_t kStagedParticles = 16384;
+
+// A staged round whose curve would take no more than this if every particle lived
+// to its last iteration comes back whole, with the end states.
+constexpr uint64_t kWholeCurveBytes = 2ull << 20;
+
+// Raw (unpruned) vertex offsets of n particles, remaining + 2 slots each, and
+// their total behind them; returns the total.
+uint64_t fill_raw_offsets(const uint64_t* remaining, uint64_t n, uint64_t* offsets) {
+  uint64_t total = 0;
   for (uint64_t i = 0; i < n; ++i) {
-    offsets[i] = raw_total;
-    raw_total += host_remaining[begin + i] + 2;
+    offsets[i] = total;
+    total += remaining[i] + 2;
   }
-  offsets[n] = raw_total;
-  DPA_TRY_CUDA(ctx, ctx->raw.reserve(raw_total * 12));
-  DPA_TRY_CUDA(ctx, ctx->raw_offsets.reserve((n + 1) * 8));
+  offsets[n] = total;
+  return total;
+}
+
+// Device arrays of n particles of a recording round: raw_offsets has n + 1
+// entries, the last of them raw_total; totals receives the kept vertices and the
+// kept segments.
+struct piece_arrays {
+  float* positions;
+  uint64_t* remaining;
+  uint8_t* termination;
+  const uint64_t* raw_offsets;
+  uint64_t raw_total;
+  unsigned long long* totals;
+};
+
+// Order, advection and curve offsets of a piece.
+int advect_curves(dpa_context* ctx, const dpa_field* field, const dpa_advect_options* o,
+                  const dpa::StepCoefficients& k, uint64_t n, const piece_arrays& p) {
+  cudaStream_t s = ctx->stream;
+  DPA_TRY_CUDA(ctx, ctx->raw.reserve(p.raw_total * 12));
   DPA_TRY_CUDA(ctx, ctx->kept_vertices.reserve(n * 4));
   DPA_TRY_CUDA(ctx, ctx->kept_segments.reserve(n * 4));
   DPA_TRY_CUDA(ctx, ctx->vertex_offsets.reserve(n * 8));
   DPA_TRY_CUDA(ctx, ctx->segment_offsets.reserve(n * 8));
-  DPA_TRY_CUDA(ctx, ctx->totals.reserve(32));
-  DPA_TRY_CUDA(ctx, ctx->host_totals.reserve(32));
-  // The pinned offsets of the previous piece are free: its copies finished
-  // before the previous piece returned.
-  DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->raw_offsets.ptr, offsets, (n + 1) * 8,
-                                    cudaMemcpyHostToDevice, s));
-
-  float* positions = ctx->positions.as<float>() + 3 * begin;
-  uint64_t* remaining = ctx->remaining.as<uint64_t>() + begin;
-  uint8_t* termination = ctx->termination.as<uint8_t>() + begin;
   if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[0], s));
   const uint32_t* order = nullptr;
   if (o->morton_order && ctx->tuning.order) {
-    const int st = build_order(ctx, ctx->scratch, field, positions, n, s, &order);
+    const int st = build_order(ctx, ctx->scratch, field, p.positions, n, s, &order);
     if (st != DPA_OK) return st;
   }
   if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[1], s));
@@ -188,12 +197,12 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
   a.work_counter = ctx->scratch.work_counter.as<unsigned long long>();
   a.count = n;
   a.order = order;
-  a.positions = positions;
-  a.remaining = remaining;
-  a.termination = termination;
+  a.positions = p.positions;
+  a.remaining = p.remaining;
+  a.termination = p.termination;
   a.coefficients = k;
   a.raw_vertices = ctx->raw.as<float>();
-  a.raw_offsets = ctx->raw_offsets.as<uint64_t>();
+  a.raw_offsets = p.raw_offsets;
   a.kept_vertices = ctx->kept_vertices.as<uint32_t>();
   a.kept_segments = ctx->kept_segments.as<uint32_t>();
   DPA_TRY_CUDA(ctx, dpa::launch_advect(field->view, a, o->integrator, true, s));
@@ -202,41 +211,103 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
     DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[2], s));
     DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[3], s));
   }
-
-  // Piece-local offsets of kept vertices and kept segments and their totals.
   DPA_TRY_CUDA(ctx, ctx->scan_temp.reserve(dpa::curve_offsets_scratch_bytes(n)));
   DPA_TRY_CUDA(ctx, dpa::launch_curve_offsets(
                         ctx->kept_vertices.as<uint32_t>(), ctx->kept_segments.as<uint32_t>(), n,
                         ctx->scan_temp.ptr, ctx->vertex_offsets.as<uint64_t>(),
-                        ctx->segment_offsets.as<uint64_t>(),
-                        ctx->totals.as<unsigned long long>(), s));
+                        ctx->segment_offsets.as<uint64_t>(), p.totals, s));
   ctx->launches += uint64_t(dpa::curve_offsets_launches(n));
-  uint64_t* ht = ctx->host_totals.as<uint64_t>();
-  DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ht, ctx->totals.ptr, 16, cudaMemcpyDeviceToHost, s));
-  const size_t index_bytes = o->index64 ? 8 : 4;
-  // A small piece is emitted without waiting for its totals, into room for all
-  // of its raw vertices; a large one waits, and takes no more than it needs.
-  const bool early = raw_total * 12 <= kEarlyEmitBytes;
-  if (!early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
-  DPA_TRY_CUDA(ctx, ctx->out_vertices.reserve((early ? raw_total : ht[0]) * 12));
-  DPA_TRY_CUDA(ctx, ctx->out_colors.reserve((early ? raw_total : ht[0]) * 4));
-  DPA_TRY_CUDA(ctx, ctx->out_indices.reserve(2 * (early ? raw_total : ht[1]) * index_bytes));
+  return DPA_OK;
+}
 
+// The piece's pruned curve, index pairs and colors.
+int emit_curves(dpa_context* ctx, const dpa_advect_options* o, uint64_t n, const piece_arrays& p,
+                uint64_t vertex_base, float* vertices, float* colors, void* indices) {
   dpa::EmitArgs e{};
   e.count = n;
   e.raw_vertices = ctx->raw.as<float>();
-  e.raw_offsets = ctx->raw_offsets.as<uint64_t>();
-  e.remaining = remaining;
+  e.raw_offsets = p.raw_offsets;
+  e.remaining = p.remaining;
   e.vertex_offsets = ctx->vertex_offsets.as<uint64_t>();
   e.segment_offsets = ctx->segment_offsets.as<uint64_t>();
   e.kept_vertices = ctx->kept_vertices.as<uint32_t>();
-  e.vertex_base = *round_vertices;
-  e.vertices = ctx->out_vertices.as<float>();
-  e.colors = o->colors ? ctx->out_colors.as<float>() : nullptr;
-  e.indices = ctx->out_indices.ptr;
-  DPA_TRY_CUDA(ctx, dpa::launch_emit(e, o->index64 != 0, o->colors != 0, s));
+  e.vertex_base = vertex_base;
+  e.vertices = vertices;
+  e.colors = o->colors ? colors : nullptr;
+  e.indices = indices;
+  DPA_TRY_CUDA(ctx, dpa::launch_emit(e, o->index64 != 0, o->colors != 0, ctx->stream));
   ctx->launches += 1;
-  if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[4], s));
+  if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[4], ctx->stream));
+  return DPA_OK;
+}
+
+// A round's arrays in one block, on the device and, for a staged round, in pinned
+// memory: a staged round's inputs (raw offsets, positions, remaining) go in by one
+// copy and its results (positions to totals and, for a round that comes back whole,
+// its curve) return by one.
+struct round_arrays {
+  uint64_t offsets, positions, remaining, termination, totals, vertices, colors, indices, bytes;
+
+  round_arrays(uint64_t count, uint64_t offset_entries, uint64_t curve_vertices,
+               size_t index_bytes) {
+    bytes = 0;
+    auto place = [this](uint64_t size) {
+      const uint64_t at = bytes;
+      bytes += (size + 15) / 16 * 16;
+      return at;
+    };
+    offsets = place(offset_entries * 8);
+    positions = place(count * 12);
+    remaining = place(count * 8);
+    termination = place(count);
+    totals = place(16);
+    vertices = place(curve_vertices * 12);
+    colors = place(curve_vertices * 4);
+    indices = place(2 * curve_vertices * index_bytes);
+  }
+};
+
+// Advects and emits particles [begin, end) of a recording round, whose device
+// arrays start at `round`.
+int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_options* o,
+                 const dpa::StepCoefficients& k, uint64_t begin, uint64_t end,
+                 const piece_arrays& round, const uint64_t* host_remaining,
+                 uint64_t* round_vertices, uint64_t* round_indices, bool final_piece,
+                 dpa_curve_sink sink, void* user) {
+  cudaStream_t s = ctx->stream;
+  const uint64_t n = end - begin;
+  piece_arrays p = round;
+  p.positions += 3 * begin;
+  p.remaining += begin;
+  p.termination += begin;
+  if (!p.raw_offsets) {
+    // Raw (unpruned) vertex offsets: remaining + 2 slots per particle.
+    DPA_TRY_CUDA(ctx, ctx->host_offsets.reserve((n + 1) * 8));
+    DPA_TRY_CUDA(ctx, ctx->raw_offsets.reserve((n + 1) * 8));
+    // The pinned offsets of the previous piece are free: its copies finished
+    // before the previous piece returned.
+    uint64_t* offsets = ctx->host_offsets.as<uint64_t>();
+    p.raw_total = fill_raw_offsets(host_remaining + begin, n, offsets);
+    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->raw_offsets.ptr, offsets, (n + 1) * 8,
+                                      cudaMemcpyHostToDevice, s));
+    p.raw_offsets = ctx->raw_offsets.as<uint64_t>();
+  }
+  DPA_TRY_CUDA(ctx, ctx->host_totals.reserve(32));
+  int st = advect_curves(ctx, field, o, k, n, p);
+  if (st != DPA_OK) return st;
+  uint64_t* ht = ctx->host_totals.as<uint64_t>();
+  DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ht, p.totals, 16, cudaMemcpyDeviceToHost, s));
+  const size_t index_bytes = o->index64 ? 8 : 4;
+  // A small piece is emitted without waiting for its totals, into room for all
+  // of its raw vertices; a large one waits, and takes no more than it needs.
+  const bool early = p.raw_total * 12 <= kEarlyEmitBytes;
+  if (!early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+  DPA_TRY_CUDA(ctx, ctx->out_vertices.reserve((early ? p.raw_total : ht[0]) * 12));
+  DPA_TRY_CUDA(ctx, ctx->out_colors.reserve((early ? p.raw_total : ht[0]) * 4));
+  DPA_TRY_CUDA(ctx, ctx->out_indices.reserve(2 * (early ? p.raw_total : ht[1]) * index_bytes));
+  st = emit_curves(ctx, o, n, p, *round_vertices, ctx->out_vertices.as<float>(),
+                   ctx->out_colors.as<float>(), ctx->out_indices.ptr);
+  if (st != DPA_OK) return st;
   if (early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
   const uint64_t piece_vertices = ht[0];
   const uint64_t piece_segments = ht[1];
@@ -246,30 +317,39 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
                 "the round's curve has more vertices than 32-bit indices can address; "
                 "set index64");
 
-  // The piece's curve crosses to the host in chunks through two pinned
-  // halves, so that chunk j + 1 copies while the sink takes chunk j and the
-  // pinned memory stays bounded (dpa_context_set_host_chunk_limit).
+  // The piece's curve crosses to the host in chunks through two pinned halves, so
+  // that a chunk copies while the sink takes the one before it and the pinned memory
+  // stays bounded (dpa_context_set_host_chunk_limit). Chunks begin at 1 MiB of
+  // vertices and colors, which with its indices stays in a core's 2 MiB cache while
+  // the sink copies it on (260 MB in three rounds into the caller's arrays: 22.6 ms,
+  // against 24 to 25 at 2 MiB or in one chunk and 27.9 at 16 MiB), and double, to
+  // 16 MiB at most, whenever the next one had not landed when the sink returned: the
+  // copies then bound the round, and larger ones cost less (the same rounds,
+  // discarded: 6.4 ms in chunks of 1 MiB, 5.2 doubling).
   if (sink) {
-    const uint64_t cap_v = std::max<uint64_t>(ctx->host_chunk_bytes / 16, 1);
-    const uint64_t cap_i = std::max<uint64_t>(ctx->host_chunk_bytes / index_bytes, 2) & ~1ull;
-    const uint64_t chunks = std::max<uint64_t>(
-        {1, (piece_vertices + cap_v - 1) / cap_v, (piece_indices + cap_i - 1) / cap_i});
-    const uint64_t half_v = std::min(piece_vertices, cap_v);
-    const uint64_t half_i = std::min(piece_indices, cap_i);
+    constexpr uint64_t kFirstChunk = 1ull << 20, kMostChunk = 16ull << 20;
+    const uint64_t most_v = std::max<uint64_t>(std::min(ctx->host_chunk_bytes, kMostChunk) / 16, 1);
+    const uint64_t most_i = std::max<uint64_t>(ctx->host_chunk_bytes / index_bytes, 2) & ~1ull;
+    uint64_t cap_v = std::min(most_v, kFirstChunk / 16);
+    auto cap_i = [&] { return std::min(most_i, 2 * cap_v); };
+    const uint64_t half_v = std::min(piece_vertices, most_v);
+    const uint64_t half_i = std::min({piece_indices, most_i, 2 * most_v});
     DPA_TRY_CUDA(ctx, ctx->host_vertices.reserve(2 * half_v * 12));
     DPA_TRY_CUDA(ctx, ctx->host_colors.reserve(2 * half_v * 4));
     DPA_TRY_CUDA(ctx, ctx->host_indices.reserve(2 * half_i * index_bytes));
     for (cudaEvent_t& ev : ctx->chunk_events)
       if (!ev) DPA_TRY_CUDA(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    auto span = [](uint64_t j, uint64_t cap, uint64_t total, uint64_t* first, uint64_t* count) {
-      *first = std::min(j * cap, total);
-      *count = std::min(cap, total - *first);
-    };
-    auto issue = [&](uint64_t j) -> int {
-      const uint64_t h = j & 1;
+    struct {
       uint64_t v0, vn, i0, in;
-      span(j, cap_v, piece_vertices, &v0, &vn);
-      span(j, cap_i, piece_indices, &i0, &in);
+    } span[2];
+    uint64_t next_v = 0, next_i = 0;
+    auto all_issued = [&] { return next_v == piece_vertices && next_i == piece_indices; };
+    auto issue = [&](uint64_t h) -> int {  // the next chunk, into half h
+      span[h] = {next_v, std::min(cap_v, piece_vertices - next_v), next_i,
+                 std::min(cap_i(), piece_indices - next_i)};
+      const auto [v0, vn, i0, in] = span[h];
+      next_v += vn;
+      next_i += in;
       if (vn) {
         DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->host_vertices.as<float>() + 3 * h * half_v,
                                           ctx->out_vertices.as<float>() + 3 * v0, vn * 12,
@@ -287,27 +367,31 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
       DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->chunk_events[h], s));
       return DPA_OK;
     };
-    int st = issue(0);
+    st = issue(0);
     if (st != DPA_OK) return st;
-    for (uint64_t j = 0; j < chunks; ++j) {
-      if (j + 1 < chunks) {
-        st = issue(j + 1);  // into the half whose chunk the sink has returned
+    bool more = true;
+    for (uint64_t h = 0; more; h ^= 1) {
+      more = !all_issued();
+      if (more) {
+        st = issue(h ^ 1);  // into the half whose chunk the sink has returned
         if (st != DPA_OK) return st;
       }
-      const uint64_t h = j & 1;
-      DPA_TRY_CUDA(ctx, cudaEventSynchronize(ctx->chunk_events[h]));
-      uint64_t v0, vn, i0, in;
-      span(j, cap_v, piece_vertices, &v0, &vn);
-      span(j, cap_i, piece_indices, &i0, &in);
+      const cudaError_t landed = cudaEventQuery(ctx->chunk_events[h]);
+      if (landed == cudaErrorNotReady) {
+        if (span[h].v0) cap_v = std::min(2 * cap_v, most_v);
+        DPA_TRY_CUDA(ctx, cudaEventSynchronize(ctx->chunk_events[h]));
+      } else {
+        DPA_TRY_CUDA(ctx, landed);
+      }
       dpa_curve_chunk c{};
-      c.vertex_offset = *round_vertices + v0;
-      c.vertex_count = vn;
+      c.vertex_offset = *round_vertices + span[h].v0;
+      c.vertex_count = span[h].vn;
       c.vertices = ctx->host_vertices.as<float>() + 3 * h * half_v;
       c.colors = o->colors ? ctx->host_colors.as<float>() + h * half_v : nullptr;
-      c.index_offset = *round_indices + i0;
-      c.index_count = in;
+      c.index_offset = *round_indices + span[h].i0;
+      c.index_count = span[h].in;
       c.indices = ctx->host_indices.as<char>() + h * half_i * index_bytes;
-      c.last = (final_piece && j + 1 == chunks) ? 1 : 0;
+      c.last = (final_piece && !more) ? 1 : 0;
       if (sink(user, &c) != 0) {
         cudaStreamSynchronize(s);  // no copy may still target the halves
         return fail(ctx, DPA_ERROR_SINK, "curve sink aborted the round");
@@ -788,21 +872,58 @@ int dpa_advect_round(dpa_context* ctx, const dpa_field* field, const dpa_advect_
       }
       return DPA_OK;
     }
-    DPA_TRY_CUDA(ctx, ctx->positions.reserve(count * 12));
-    DPA_TRY_CUDA(ctx, ctx->remaining.reserve(count * 8));
-    DPA_TRY_CUDA(ctx, ctx->termination.reserve(count));
-    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->positions.ptr, positions, count * 12,
-                                      cudaMemcpyHostToDevice, s));
-    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->remaining.ptr, remaining, count * 8,
-                                      cudaMemcpyHostToDevice, s));
-    if (!options->record) {
-      st = advect_device_impl(ctx, field, options, count, ctx->positions.as<float>(),
-                              ctx->remaining.as<uint64_t>(), ctx->termination.as<uint8_t>(), s);
+    const bool record = options->record != 0;
+    const size_t index_bytes = options->index64 ? 8 : 4;
+    const uint64_t limit_vertices = std::max<uint64_t>(ctx->staging_limit / 12, 1);
+    const bool staged = count <= kStagedParticles;
+    uint64_t raw_total = 0;
+    if (record)
+      for (uint64_t i = 0; i < count && raw_total <= limit_vertices; ++i)
+        raw_total += remaining[i] + 2;
+    const bool one_piece = record && (raw_total <= limit_vertices || count == 1);
+    const uint64_t whole_bytes = raw_total * std::max<uint64_t>(16, 2 * index_bytes);
+    const bool whole = staged && one_piece && whole_bytes <= ctx->host_chunk_bytes &&
+                       raw_total * (16 + 2 * index_bytes) <= kWholeCurveBytes && !ctx->profiling;
+    const round_arrays at(count, staged && one_piece ? count + 1 : 0, whole ? raw_total : 0,
+                          index_bytes);
+    DPA_TRY_CUDA(ctx, ctx->round.reserve(at.bytes));
+    char* const device = ctx->round.as<char>();
+    char* host = nullptr;
+    piece_arrays p{};
+    p.positions = reinterpret_cast<float*>(device + at.positions);
+    p.remaining = reinterpret_cast<uint64_t*>(device + at.remaining);
+    p.termination = reinterpret_cast<uint8_t*>(device + at.termination);
+    p.totals = reinterpret_cast<unsigned long long*>(device + at.totals);
+    if (staged) {
+      DPA_TRY_CUDA(ctx, ctx->host_round.reserve(at.bytes));
+      host = ctx->host_round.as<char>();
+      if (one_piece) {
+        p.raw_offsets = reinterpret_cast<uint64_t*>(device + at.offsets);
+        p.raw_total = fill_raw_offsets(remaining, count,
+                                       reinterpret_cast<uint64_t*>(host + at.offsets));
+      }
+      std::memcpy(host + at.positions, positions, count * 12);
+      std::memcpy(host + at.remaining, remaining, count * 8);
+      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(device, host, at.termination, cudaMemcpyHostToDevice, s));
+    } else {
+      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(p.positions, positions, count * 12,
+                                        cudaMemcpyHostToDevice, s));
+      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(p.remaining, remaining, count * 8,
+                                        cudaMemcpyHostToDevice, s));
+    }
+    if (!record) {
+      st = advect_device_impl(ctx, field, options, count, p.positions, p.remaining, p.termination,
+                              s);
+      if (st != DPA_OK) return st;
+    } else if (whole) {
+      st = advect_curves(ctx, field, options, k, count, p);
+      if (st == DPA_OK)
+        st = emit_curves(ctx, options, count, p, 0, reinterpret_cast<float*>(device + at.vertices),
+                         reinterpret_cast<float*>(device + at.colors), device + at.indices);
       if (st != DPA_OK) return st;
     } else {
       ctx->round_order_ms = ctx->round_advect_ms = ctx->round_emit_ms = 0.0f;
       // Pieces of the round whose unpruned curves fit the staging limit.
-      const uint64_t limit_vertices = std::max<uint64_t>(ctx->staging_limit / 12, 1);
       uint64_t round_vertices = 0, round_indices = 0;
       uint64_t begin = 0;
       while (begin < count) {
@@ -811,7 +932,7 @@ int dpa_advect_round(dpa_context* ctx, const dpa_field* field, const dpa_advect_
           raw += remaining[end] + 2;
           ++end;
         }
-        st = record_piece(ctx, field, options, k, begin, end, remaining, &round_vertices,
+        st = record_piece(ctx, field, options, k, begin, end, p, remaining, &round_vertices,
                           &round_indices, end == count, sink, sink_user);
         if (st != DPA_OK) return st;
         begin = end;
@@ -821,13 +942,33 @@ int dpa_advect_round(dpa_context* ctx, const dpa_field* field, const dpa_advect_
         ctx->timed_order = false;
       }
     }
-    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(positions, ctx->positions.ptr, count * 12,
-                                      cudaMemcpyDeviceToHost, s));
-    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(remaining, ctx->remaining.ptr, count * 8,
-                                      cudaMemcpyDeviceToHost, s));
+    if (staged) {
+      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(host + at.positions, device + at.positions,
+                                        at.bytes - at.positions, cudaMemcpyDeviceToHost, s));
+      DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+      if (whole && sink) {
+        const uint64_t* totals = reinterpret_cast<uint64_t*>(host + at.totals);
+        dpa_curve_chunk c{};
+        c.vertex_count = totals[0];
+        c.vertices = reinterpret_cast<float*>(host + at.vertices);
+        c.colors = options->colors ? reinterpret_cast<float*>(host + at.colors) : nullptr;
+        c.index_count = 2 * totals[1];
+        c.indices = host + at.indices;
+        c.last = 1;
+        if (sink(sink_user, &c) != 0) return fail(ctx, DPA_ERROR_SINK, "curve sink aborted the round");
+      }
+      std::memcpy(positions, host + at.positions, count * 12);
+      std::memcpy(remaining, host + at.remaining, count * 8);
+      if (termination) std::memcpy(termination, host + at.termination, count);
+      return DPA_OK;
+    }
+    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(positions, p.positions, count * 12, cudaMemcpyDeviceToHost,
+                                      s));
+    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(remaining, p.remaining, count * 8, cudaMemcpyDeviceToHost,
+                                      s));
     if (termination)
-      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(termination, ctx->termination.ptr, count,
-                                        cudaMemcpyDeviceToHost, s));
+      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(termination, p.termination, count, cudaMemcpyDeviceToHost,
+                                        s));
     DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
     return DPA_OK;
   });

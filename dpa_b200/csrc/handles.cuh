@@ -115,7 +115,9 @@ struct dpa_context {
   cudaEvent_t chunk_events[2] = {nullptr, nullptr};
   bool ieee_division = false;  // fields created now divide by __fdiv_rn only
 
-  DeviceBuffer positions, remaining, remaining_in, termination;
+  DeviceBuffer round;       // a round's arrays (round_arrays, capi.cu)
+  PinnedBuffer host_round;  // a staged round's
+  DeviceBuffer remaining_in;
   dpa_launch_scratch scratch;
   uint64_t launches = 0;  // kernels this context launched (advection path)
   bool profiling = false;
@@ -127,20 +129,20 @@ struct dpa_context {
   float round_order_ms = 0.0f, round_advect_ms = 0.0f, round_emit_ms = 0.0f;
   dpa_tuning_state tuning;
   DeviceBuffer raw, raw_offsets, kept_vertices, kept_segments;
-  DeviceBuffer wide, vertex_offsets, segment_offsets, scan_temp, totals;
+  DeviceBuffer wide, vertex_offsets, segment_offsets, scan_temp;
   DeviceBuffer out_vertices, out_colors, out_indices;
   PinnedBuffer host_vertices, host_colors, host_indices, host_totals, host_offsets;
   DeviceBuffer ftle_winners, ftle_out, ftle_original, ftle_final;
 
   void release_all() {
     scratch.release();
-    DeviceBuffer* d[] = {&positions, &remaining, &remaining_in, &termination, &raw, &raw_offsets,
+    DeviceBuffer* d[] = {&round, &remaining_in, &raw, &raw_offsets,
                          &kept_vertices, &kept_segments, &wide, &vertex_offsets,
-                         &segment_offsets, &scan_temp, &totals, &out_vertices, &out_colors,
+                         &segment_offsets, &scan_temp, &out_vertices, &out_colors,
                          &out_indices, &ftle_winners, &ftle_out, &ftle_original,
                          &ftle_final};
     for (DeviceBuffer* b : d) b->release();
-    PinnedBuffer* h[] = {&host_vertices, &host_colors, &host_indices, &host_totals,
+    PinnedBuffer* h[] = {&host_round, &host_vertices, &host_colors, &host_indices, &host_totals,
                          &host_offsets};
     for (PinnedBuffer* b : h) b->release();
   }

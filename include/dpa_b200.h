@@ -161,8 +161,9 @@ int dpa_context_set_staging_limit(dpa_context* ctx, uint64_t bytes);
 
 /* Upper bound on the curve bytes one sink chunk carries (default 256 MiB of
  * vertices and colors, and as many bytes of indices). A piece's curve crosses
- * to the host through two pinned buffers of this size, the next chunk copying
- * while the sink takes the current one. */
+ * to the host through two pinned buffers, the next chunk copying while the sink
+ * takes the current one; chunks are smaller than the limit where that is faster
+ * (1 to 16 MiB of vertices and colors). */
 int dpa_context_set_host_chunk_limit(dpa_context* ctx, uint64_t bytes);
 
 /* Instrumentation, the counterpart of the reference's per-round timers
