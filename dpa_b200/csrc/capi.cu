@@ -688,11 +688,12 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     const size_t node_bytes = dpa::field_node_bytes(storage);
     for (int i = 0; i < 3; ++i) f->view.n[i] = int32_t(shape[i]);
     f->view.storage = storage;
-    cudaError_t e = f->nodes.reserve(dpa::choose_layout(f->view, slices) * node_bytes);
+    f->node_bytes = std::max<uint64_t>(dpa::choose_layout(f->view, slices) * node_bytes, 16);
+    cudaError_t e = f->nodes.reserve_from(ctx->spare, f->node_bytes);
     const float* src = xyzv;
     DeviceBuffer staging;
     if (e == cudaSuccess && !device_input) {
-      e = staging.reserve(nodes * 12);
+      e = staging.reserve_from(ctx->spare, nodes * 12);
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(staging.ptr, xyzv, nodes * 12, cudaMemcpyHostToDevice, ctx->stream);
       src = staging.as<float>();
@@ -700,6 +701,7 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     if (e == cudaSuccess)
       e = dpa::launch_repack(src, nodes, f->view, f->nodes.ptr, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) staging.release_to(ctx->spare);
     staging.release();
     if (e != cudaSuccess) {
       f->nodes.release();
@@ -822,7 +824,8 @@ int dpa_field_destroy(dpa_context* ctx, dpa_field* field) {
   if (!ctx || !field) return DPA_ERROR_INVALID_ARGUMENT;
   if (field->owner != ctx) return fail(ctx, DPA_ERROR_INVALID_ARGUMENT, "field belongs to another context");
   cudaSetDevice(ctx->device);
-  cudaStreamSynchronize(ctx->stream);
+  // Calls on any stream may still read the field; its block may be the next one's.
+  if (cudaDeviceSynchronize() == cudaSuccess) field->nodes.release_to(ctx->spare);
   field->nodes.release();
   delete field;
   return DPA_OK;
@@ -837,7 +840,7 @@ int dpa_field_info(const dpa_field* field, uint64_t shape[3], float offset[3], f
     if (spacing) spacing[i] = field->spacing[i];
   }
   if (storage) *storage = field->storage;
-  if (device_bytes) *device_bytes = field->nodes.bytes;
+  if (device_bytes) *device_bytes = field->node_bytes;
   return DPA_OK;
 }
 

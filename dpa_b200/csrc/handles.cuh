@@ -2,11 +2,87 @@
 // (dpa_context, dpa_field) and the device/pinned buffers they own.
 #pragma once
 
+#include <algorithm>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "kernels.cuh"
 
 namespace dpa {
+
+// Device blocks of destroyed fields, kept for the next field of about their size:
+// a program that makes a field of each time step would otherwise spend more on
+// allocating and freeing it than on using it. At most kKeep bytes in kMost blocks
+// stay; the oldest go first, all when the context goes or when an allocation of any
+// context of the process finds no memory. Blocks are given back only when the device
+// has finished with them.
+class SpareBlocks {
+ public:
+  static constexpr size_t kKeep = size_t(1) << 30, kMost = 4;
+  SpareBlocks() {
+    std::lock_guard<std::mutex> guard(registry().lock);
+    registry().all.push_back(this);
+  }
+  ~SpareBlocks() {
+    std::lock_guard<std::mutex> guard(registry().lock);
+    auto& all = registry().all;
+    all.erase(std::remove(all.begin(), all.end(), this), all.end());
+    release();
+  }
+  SpareBlocks(const SpareBlocks&) = delete;
+  SpareBlocks& operator=(const SpareBlocks&) = delete;
+
+  // A kept block of n bytes or up to an eighth more, or null.
+  void* take(size_t n, size_t* bytes) {
+    std::lock_guard<std::mutex> guard(lock_);
+    for (size_t i = 0; i < blocks_.size(); ++i) {
+      if (blocks_[i].bytes < n || blocks_[i].bytes - n > n / 8) continue;
+      void* ptr = blocks_[i].ptr;
+      *bytes = blocks_[i].bytes;
+      blocks_.erase(blocks_.begin() + long(i));
+      return ptr;
+    }
+    return nullptr;
+  }
+  void give(void* ptr, size_t bytes) {
+    std::lock_guard<std::mutex> guard(lock_);
+    blocks_.push_back({ptr, bytes});
+    size_t held = 0;
+    for (const block& b : blocks_) held += b.bytes;
+    while (!blocks_.empty() && (held > kKeep || blocks_.size() > kMost)) {
+      held -= blocks_.front().bytes;
+      cudaFree(blocks_.front().ptr);
+      blocks_.erase(blocks_.begin());
+    }
+  }
+  void release() {
+    std::lock_guard<std::mutex> guard(lock_);
+    for (const block& b : blocks_) cudaFree(b.ptr);
+    blocks_.clear();
+  }
+  // Returns what every context of the process keeps.
+  static void release_everywhere() {
+    std::lock_guard<std::mutex> guard(registry().lock);
+    for (SpareBlocks* s : registry().all) s->release();
+  }
+
+ private:
+  struct block {
+    void* ptr;
+    size_t bytes;
+  };
+  struct registry_type {
+    std::mutex lock;
+    std::vector<SpareBlocks*> all;
+  };
+  static registry_type& registry() {
+    static registry_type* r = new registry_type;  // outlives every context
+    return *r;
+  }
+  std::mutex lock_;
+  std::vector<block> blocks_;
+};
 
 // Grow-only device buffer; freed by release() or when it goes out of scope
 // (with its device current).
@@ -22,12 +98,28 @@ struct DeviceBuffer {
     release();
     if (n == 0) n = 16;
     cudaError_t e = cudaMalloc(&ptr, n);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      SpareBlocks::release_everywhere();
+      e = cudaMalloc(&ptr, n);
+    }
     if (e != cudaSuccess) {
       ptr = nullptr;
       return e;
     }
     bytes = n;
     return cudaSuccess;
+  }
+  // reserve() from the spare blocks where one fits, and release() to them.
+  cudaError_t reserve_from(SpareBlocks& spare, size_t n) {
+    release();
+    if (n) ptr = spare.take(n, &bytes);
+    return ptr ? cudaSuccess : reserve(n);
+  }
+  void release_to(SpareBlocks& spare) {
+    if (ptr) spare.give(ptr, bytes);
+    ptr = nullptr;
+    bytes = 0;
   }
   void release() {
     if (ptr) cudaFree(ptr);
@@ -70,6 +162,7 @@ struct PinnedBuffer {
 
 using dpa::DeviceBuffer;
 using dpa::PinnedBuffer;
+using dpa::SpareBlocks;
 
 // Launch parameters an autotuner may change per context.
 struct dpa_tuning_state {
@@ -115,6 +208,7 @@ struct dpa_context {
   cudaEvent_t chunk_events[2] = {nullptr, nullptr};
   bool ieee_division = false;  // fields created now divide by __fdiv_rn only
 
+  SpareBlocks spare;  // of destroyed fields
   DeviceBuffer round;       // a round's arrays (round_arrays, capi.cu)
   PinnedBuffer host_round;  // a staged round's
   DeviceBuffer remaining_in;
@@ -136,6 +230,7 @@ struct dpa_context {
 
   void release_all() {
     scratch.release();
+    spare.release();
     DeviceBuffer* d[] = {&round, &remaining_in, &raw, &raw_offsets,
                          &kept_vertices, &kept_segments, &wide, &vertex_offsets,
                          &segment_offsets, &scan_temp, &out_vertices, &out_colors,
@@ -151,6 +246,7 @@ struct dpa_context {
 struct dpa_field {
   dpa_context* owner = nullptr;
   DeviceBuffer nodes;
+  uint64_t node_bytes = 0;  // of nodes, a kept block being up to an eighth larger
   dpa::FieldView view{};
   uint64_t shape[3] = {0, 0, 0};
   float offset[3] = {0, 0, 0};
