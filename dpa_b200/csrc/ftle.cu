@@ -98,22 +98,23 @@ __device__ __noinline__ double max_eigenvalue_jacobi(double a[3][3]) {
 // the other two, sqrt(3 - 3/4 x^2). The gap loses digits as it closes:
 // 1 + r = 1e-8 leaves a relative error of 4e-12 in the eigenvalue, far below the
 // 6e-8 of the 32-bit result. Closer than that (a double largest eigenvalue) and
-// for matrices that are not finite the Jacobi rotations answer.
+// for matrices that are not finite it returns false: the Jacobi rotations answer.
 //
 // The rotations throughout took 1900 warp instructions for 32 cells, 800 of them in
-// 64 bits: 132 us for 1.5 million cells at 70 % of the issue slots; this takes 480
-// and 32 us.
-__device__ __forceinline__ double max_eigenvalue(double a[3][3]) {
+// 64 bits: 132 us for 1.5 million cells at 70 % of the issue slots; this took 480
+// and 32 us, and 430 and 27 us with the divisions of cauchy_green().
+__device__ __forceinline__ bool max_eigenvalue(const double a[3][3], double& largest) {
   const double q = (a[0][0] + a[1][1] + a[2][2]) * (1.0 / 3.0);
   const double b0 = a[0][0] - q, b1 = a[1][1] - q, b2 = a[2][2] - q;
   const double u = a[0][1], v = a[0][2], w = a[1][2];
   const double p2 = (b0 * b0 + b1 * b1 + b2 * b2 + 2.0 * (u * u + v * v + w * w)) * (1.0 / 6.0);
-  if (p2 == 0.0) return q;
+  largest = q;
+  if (p2 == 0.0) return true;
   const double inverse = rsqrt(p2), p = p2 * inverse;
   const double half_det =
       0.5 * (b0 * (b1 * b2 - w * w) - u * (u * b2 - w * v) + v * (u * w - b1 * v));
   const double r = half_det * inverse * inverse * inverse;
-  if (!(r >= -1.0 + 1e-8) || !(p2 < 1e300)) return max_eigenvalue_jacobi(a);
+  if (!(r >= -1.0 + 1e-8) || !(p2 < 1e300)) return false;
   const double two_r = fmin(2.0 * fabs(r), 2.0);
   constexpr float kRoot3 = 1.7320508f;
   float x0 = fmaf(0.5f * (2.0f - kRoot3), float(two_r), kRoot3);
@@ -127,34 +128,45 @@ __device__ __forceinline__ double max_eigenvalue(double a[3][3]) {
 #pragma unroll
   for (int i = 0; i < 2; ++i) x -= fma(fma(x, x, -3.0), x, -two_r) * double(slope);
   if (r < 0.0) x = 0.5 * x + sqrt(fmax(fma(-0.75 * x, x, 3.0), 0.0));
-  return fma(p, x, q);
+  largest = fma(p, x, q);
+  return true;
 }
 
-// Per lattice cell: J[r][d] = (flow[next_d] - flow[prev_d])[r] / (2 h_d) with
-// prev/next clamped at the border while the divisor stays 2 h_d; C = J^T J in
-// FP32 (Eigen's 3x3 lazy product, c0 + (c1 + c2)); the eigenvalue and the
-// logarithm in FP64. kSize holds a cell index: 32-bit divisions unless the
-// lattice needs more. The neighbours come straight from the particles' final
-// positions (a pass that laid the flow map out first took 9 to 14 us more).
-template <class kIndex, class kSize>
-__global__ void __launch_bounds__(128) ftle_kernel(const FtleArgs a, uint64_t cells) {
-  const uint64_t flat = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (flat >= cells) return;
-  const kSize n[3] = {kSize(a.shape[0]), kSize(a.shape[1]), kSize(a.shape[2])};
-  const kSize row = kSize(flat) / n[2];
-  const kSize sub[3] = {row / n[1], row % n[1], kSize(flat) - row * n[2]};
+// C = J^T J of a lattice cell in FP32 (Eigen's 3x3 lazy product, c0 + (c1 + c2)),
+// widened: J[r][d] = (flow[next_d] - flow[prev_d])[r] / (2 h_d) with prev/next
+// clamped at the border (bit d of `border`: no cell before this one along d, bit
+// 3 + d: none behind it) while the divisor stays 2 h_d. The neighbours come straight
+// from the particles' final positions (a pass that laid the flow map out first took
+// 9 to 14 us more).
+//
+// kReciprocal divides by a product with the rounded reciprocal and one correction by
+// its remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000", IBM J. Res. Dev. 34(1), 1990): 3 instructions instead of about 10,
+// nine times a cell. Its quotients are IEEE's while the remainder's last bits are
+// representable; where they are not (differences below 2^-101) the squares vanish in
+// FP32 for the divisors it is used with, [2^-26, 2^26]. Infinities come out as NaN,
+// which sends the cell to the other form.
+template <class kIndex, bool kReciprocal>
+__device__ __forceinline__ void cauchy_green(const FtleArgs& a, uint64_t flat, unsigned border,
+                                             double C[3][3]) {
   const uint64_t step[3] = {a.shape[1] * a.shape[2], a.shape[2], 1};
   float J[3][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     float prev[3], next[3];
-    flow_at<kIndex>(a, sub[d] > 0 ? flat - step[d] : flat, prev);
-    flow_at<kIndex>(a, sub[d] + 1 < n[d] ? flat + step[d] : flat, next);
+    flow_at<kIndex>(a, border >> d & 1u ? flat : flat - step[d], prev);
+    flow_at<kIndex>(a, border >> (3 + d) & 1u ? flat : flat + step[d], next);
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
-      J[r][d] = __fdiv_rn(__fsub_rn(next[r], prev[r]), a.two_spacing[d]);
+    for (int r = 0; r < 3; ++r) {
+      const float n = __fsub_rn(next[r], prev[r]);
+      if constexpr (kReciprocal) {
+        const float q = __fmul_rn(n, a.reciprocal[d]);
+        J[r][d] = __fmaf_rn(__fmaf_rn(-q, a.two_spacing[d], n), a.reciprocal[d], q);
+      } else {
+        J[r][d] = __fdiv_rn(n, a.two_spacing[d]);
+      }
+    }
   }
-  double C[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -162,15 +174,53 @@ __global__ void __launch_bounds__(128) ftle_kernel(const FtleArgs a, uint64_t ce
       C[i][j] = C[j][i] =
           double(__fadd_rn(__fmul_rn(J[0][i], J[0][j]),
                            __fadd_rn(__fmul_rn(J[1][i], J[1][j]), __fmul_rn(J[2][i], J[2][j]))));
-  a.ftle[flat] = float(0.5 * log(max_eigenvalue(C)) * a.inverse_horizon);
+}
+
+// The cells that the closed form leaves.
+template <class kIndex>
+__device__ __noinline__ double max_eigenvalue_general(const FtleArgs& a, uint64_t flat,
+                                                      unsigned border) {
+  double C[3][3];
+  cauchy_green<kIndex, false>(a, flat, border, C);
+  return max_eigenvalue_jacobi(C);
+}
+
+// The eigenvalue and the logarithm in FP64. kSize holds a cell index: 32-bit
+// divisions unless the lattice needs more.
+template <class kIndex, class kSize, bool kReciprocal>
+__global__ void __launch_bounds__(128) ftle_kernel(const __grid_constant__ FtleArgs a,
+                                                   uint64_t cells) {
+  const uint64_t flat = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (flat >= cells) return;
+  const kSize n[3] = {kSize(a.shape[0]), kSize(a.shape[1]), kSize(a.shape[2])};
+  const kSize row = kSize(flat) / n[2];
+  const kSize sub[3] = {row / n[1], row % n[1], kSize(flat) - row * n[2]};
+  unsigned border = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    border |= (sub[d] == 0 ? 1u << d : 0u) | (sub[d] + 1 == n[d] ? 8u << d : 0u);
+  double C[3][3], largest;
+  cauchy_green<kIndex, kReciprocal>(a, flat, border, C);
+  if (!max_eigenvalue(C, largest)) largest = max_eigenvalue_general<kIndex>(a, flat, border);
+  a.ftle[flat] = float(0.5 * log(largest) * a.inverse_horizon);
+}
+
+template <class kIndex, bool kReciprocal>
+cudaError_t launch_ftle_kernel(const FtleArgs& a, uint64_t cells, cudaStream_t stream) {
+  const unsigned blocks = blocks_for(cells, 128);
+  if (cells <= 0xffffffffull)
+    ftle_kernel<kIndex, uint32_t, kReciprocal><<<blocks, 128, 0, stream>>>(a, cells);
+  else
+    ftle_kernel<kIndex, uint64_t, kReciprocal><<<blocks, 128, 0, stream>>>(a, cells);
+  return cudaGetLastError();
 }
 
 template <class kIndex>
 cudaError_t launch_ftle_cells(const FtleArgs& a, uint64_t cells, cudaStream_t stream) {
-  const unsigned blocks = blocks_for(cells, 128);
-  if (cells <= 0xffffffffull) ftle_kernel<kIndex, uint32_t><<<blocks, 128, 0, stream>>>(a, cells);
-  else ftle_kernel<kIndex, uint64_t><<<blocks, 128, 0, stream>>>(a, cells);
-  return cudaGetLastError();
+  bool reciprocal = true;
+  for (float h : a.two_spacing) reciprocal = reciprocal && h >= 0x1p-26f && h <= 0x1p26f;
+  return reciprocal ? launch_ftle_kernel<kIndex, true>(a, cells, stream)
+                    : launch_ftle_kernel<kIndex, false>(a, cells, stream);
 }
 
 template <class kIndex>
@@ -230,6 +280,7 @@ cudaError_t launch_random_seeds(const float offset[3], const float size[3], uint
 cudaError_t launch_ftle(const FtleArgs& args, cudaStream_t stream) {
   FtleArgs a = args;
   a.inverse_horizon = 1.0 / a.horizon;
+  for (int i = 0; i < 3; ++i) a.reciprocal[i] = 1.0f / a.two_spacing[i];
   const uint64_t cells = a.shape[0] * a.shape[1] * a.shape[2];
   if (cells == 0) return cudaSuccess;
   if (a.mapping == DPA_FTLE_MAPPING_LATTICE) return launch_ftle_cells<void>(a, cells, stream);

@@ -202,7 +202,8 @@ struct FtleArgs {
   float spacing[3];        // field spacing * stride
   float two_spacing[3];
   double horizon;          // |step_size * iterations| as the reference rounds it
-  double inverse_horizon;  // set by the launcher
+  double inverse_horizon;  // 1 / horizon, set by the launcher
+  float reciprocal[3];     // 1 / two_spacing, set by the launcher
   void* winners;           // scratch of the reference mapping, 8 bytes a cell
   float* ftle;             // [cells]
 };

@@ -31,11 +31,12 @@ def _final(kind, x, rng):
     return out
 
 
+@pytest.mark.parametrize("spacing", [(0.7, 1.0, 0.3), (1e-9, 0.7, 1e9)])
 @pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 5), (7, 3, 33), (16, 13, 129)])
 @pytest.mark.parametrize("kind", ["identity", "double", "nearly", "zero", "noise", "not finite"])
-def test_ftle_cells(ctx, kind, shape):
+def test_ftle_cells(ctx, kind, shape, spacing):
     rng = np.random.default_rng(sum(shape))
-    grid = dpa_b200.RegularGrid.from_data(np.zeros(shape + (3,), np.float32), (0.7, 1.0, 0.3))
+    grid = dpa_b200.RegularGrid.from_data(np.zeros(shape + (3,), np.float32), spacing)
     field = ctx.field(grid)
     i = np.stack(np.meshgrid(*map(np.arange, shape), indexing="ij"), -1).reshape(-1, 3)
     x = (i.astype(np.float32) * grid.spacing).astype(np.float32)
