@@ -54,8 +54,8 @@ constexpr int advect_min_blocks() {
 // later launch.
 //
 // Between hand-outs the warp runs stretches: every slot steps until one of
-// the warp's particles stops, with one vote per step and a 32-bit step
-// counter per stretch (a stretch ends at 2^32 - 1 steps at the latest). The
+// the warp's particles stops or has no step left, with one vote per step and one
+// count for the warp (a stretch ends at 2^32 - 1 steps at the latest). The
 // kPPT slots of a lane step in lock-step, so one particle's corner gather is
 // in flight while the other's arithmetic issues. An empty slot holds a parked
 // position, the centre of the first cell (never NaN, which would send the
@@ -199,21 +199,19 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
       continue;  // every lane drew a finished particle (serving): claim again
     }
 
-    // One stretch.
-    uint32_t it[kPPT], limit[kPPT];
+    // One stretch: as many steps as every particle of the warp may still take.
+    uint32_t steps = 0xffffffffu;
     int r[kPPT];
-    bool stop[kPPT];
-    bool halt = false;
 #pragma unroll
     for (int j = 0; j < kPPT; ++j) {
-      const uint64_t allowed = active[j] ? budget[j][tid] : 0;
-      limit[j] = allowed < 0xffffffffull ? uint32_t(allowed) : 0xffffffffu;
-      it[j] = 0;
+      const uint64_t allowed = active[j] ? budget[j][tid] : ~0ull;
+      steps = allowed < steps ? uint32_t(allowed) : steps;
       r[j] = kStepTaken;
-      stop[j] = active[j] && limit[j] == 0;
-      halt = halt || stop[j];
     }
-    while (!__any_sync(kFull, halt)) {
+    steps = __reduce_min_sync(kFull, steps);
+    uint32_t n = 0;
+    bool halt = false;
+    while (n != steps && !halt) {
       // Branch-free steppers run every slot, an empty one without moving it;
       // the others skip empty slots.
 #pragma unroll
@@ -226,16 +224,15 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
                      ? step<kIntegrator>(f, a.coefficients, sampler[j], p[j], t[j], history[j])
                      : int(kStepOutOfBounds);
       }
-      halt = false;
+      ++n;
 #pragma unroll
       for (int j = 0; j < kPPT; ++j) {
         const bool taken = r[j] == kStepTaken;  // never for an empty slot
-        it[j] += taken ? 1u : 0u;
         if constexpr (kUnsteady) t[j] = taken ? __fadd_rn(t[j], a.coefficients.dt) : t[j];
         if constexpr (kRecord) {
           // The step's vertex, stored by predicated stores rather than a
           // branch (a launch of few particles waits on each step's chain).
-          float* v = curve[j] + 3 * uint64_t(it[j]);
+          float* v = curve[j] + 3 * uint64_t(n);
           asm volatile(
               "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
               "@p st.global.f32 [%0], %1;\n\t@p st.global.f32 [%0+4], %2;\n\t"
@@ -243,16 +240,17 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
               "f"(p[j].p0), "f"(p[j].p21.y), "f"(p[j].p21.x), "r"(taken ? 1u : 0u));
           counter[j].append(p[j].p0, p[j].p21.y, p[j].p21.x, taken);
         }
-        stop[j] = !taken || it[j] >= limit[j];
-        halt = halt || (active[j] && stop[j]);
+        halt = halt || (active[j] && !taken);
       }
+      halt = __any_sync(kFull, halt);
     }
 
 #pragma unroll
     for (int j = 0; j < kPPT; ++j) {
       if (!active[j]) continue;
-      const uint64_t rem = remaining[j][tid] - it[j];
-      const uint64_t left = budget[j][tid] - it[j];
+      const uint32_t taken = r[j] == kStepTaken ? n : n - 1;
+      const uint64_t rem = remaining[j][tid] - taken;
+      const uint64_t left = budget[j][tid] - taken;
       remaining[j][tid] = rem;
       budget[j][tid] = left;
       if constexpr (!kUnsteady) {
@@ -260,11 +258,11 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
         // advances by dt per step taken, rounded step by step as a
         // time-varying field's does.
         if (a.times)
-          for (uint32_t i = 0; i < it[j]; ++i) t[j] = __fadd_rn(t[j], a.coefficients.dt);
+          for (uint32_t i = 0; i < taken; ++i) t[j] = __fadd_rn(t[j], a.coefficients.dt);
       }
-      if constexpr (kRecord) curve[j] += 3 * uint64_t(it[j]);
+      if constexpr (kRecord) curve[j] += 3 * uint64_t(taken);
       // A particle that only reached the end of a stretch carries on.
-      if (!stop[j] || (r[j] == kStepTaken && left > 0)) continue;
+      if (r[j] == kStepTaken && left > 0) continue;
 
       const uint64_t k = particle[j][tid];
       const int reason = r[j] == kStepOutOfBounds    ? DPA_TERMINATION_OUT_OF_BOUNDS
