@@ -174,15 +174,15 @@ struct piece_arrays {
   unsigned long long* totals;
 };
 
-// Order, advection and curve offsets of a piece.
+// Order, advection and, unless the emission does without them, curve offsets of a
+// piece.
 int advect_curves(dpa_context* ctx, const dpa_field* field, const dpa_advect_options* o,
-                  const dpa::StepCoefficients& k, uint64_t n, const piece_arrays& p) {
+                  const dpa::StepCoefficients& k, uint64_t n, const piece_arrays& p,
+                  bool scans) {
   cudaStream_t s = ctx->stream;
   DPA_TRY_CUDA(ctx, ctx->raw.reserve(p.raw_total * 12));
   DPA_TRY_CUDA(ctx, ctx->kept_vertices.reserve(n * 4));
   DPA_TRY_CUDA(ctx, ctx->kept_segments.reserve(n * 4));
-  DPA_TRY_CUDA(ctx, ctx->vertex_offsets.reserve(n * 8));
-  DPA_TRY_CUDA(ctx, ctx->segment_offsets.reserve(n * 8));
   if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[0], s));
   const uint32_t* order = nullptr;
   if (o->morton_order && ctx->tuning.order) {
@@ -211,6 +211,9 @@ int advect_curves(dpa_context* ctx, const dpa_field* field, const dpa_advect_opt
     DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[2], s));
     DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[3], s));
   }
+  if (!scans) return DPA_OK;
+  DPA_TRY_CUDA(ctx, ctx->vertex_offsets.reserve(n * 8));
+  DPA_TRY_CUDA(ctx, ctx->segment_offsets.reserve(n * 8));
   DPA_TRY_CUDA(ctx, ctx->scan_temp.reserve(dpa::curve_offsets_scratch_bytes(n)));
   DPA_TRY_CUDA(ctx, dpa::launch_curve_offsets(
                         ctx->kept_vertices.as<uint32_t>(), ctx->kept_segments.as<uint32_t>(), n,
@@ -220,16 +223,21 @@ int advect_curves(dpa_context* ctx, const dpa_field* field, const dpa_advect_opt
   return DPA_OK;
 }
 
-// The piece's pruned curve, index pairs and colors.
+// The piece's pruned curve, index pairs and colors (and, without scans, its totals).
 int emit_curves(dpa_context* ctx, const dpa_advect_options* o, uint64_t n, const piece_arrays& p,
-                uint64_t vertex_base, float* vertices, float* colors, void* indices) {
+                bool scans, uint64_t vertex_base, float* vertices, float* colors,
+                void* indices) {
   dpa::EmitArgs e{};
   e.count = n;
   e.raw_vertices = ctx->raw.as<float>();
   e.raw_offsets = p.raw_offsets;
   e.remaining = p.remaining;
-  e.vertex_offsets = ctx->vertex_offsets.as<uint64_t>();
-  e.segment_offsets = ctx->segment_offsets.as<uint64_t>();
+  if (scans) {
+    e.vertex_offsets = ctx->vertex_offsets.as<uint64_t>();
+    e.segment_offsets = ctx->segment_offsets.as<uint64_t>();
+  }
+  e.totals = p.totals;
+  e.kept_segments = ctx->kept_segments.as<uint32_t>();
   e.kept_vertices = ctx->kept_vertices.as<uint32_t>();
   e.vertex_base = vertex_base;
   e.vertices = vertices;
@@ -293,22 +301,27 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
     p.raw_offsets = ctx->raw_offsets.as<uint64_t>();
   }
   DPA_TRY_CUDA(ctx, ctx->host_totals.reserve(32));
-  int st = advect_curves(ctx, field, o, k, n, p);
-  if (st != DPA_OK) return st;
-  uint64_t* ht = ctx->host_totals.as<uint64_t>();
-  DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ht, p.totals, 16, cudaMemcpyDeviceToHost, s));
   const size_t index_bytes = o->index64 ? 8 : 4;
   // A small piece is emitted without waiting for its totals, into room for all
   // of its raw vertices; a large one waits, and takes no more than it needs.
   const bool early = p.raw_total * 12 <= kEarlyEmitBytes;
-  if (!early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+  const bool scans = !early || n > dpa::kEmitScans;
+  int st = advect_curves(ctx, field, o, k, n, p, scans);
+  if (st != DPA_OK) return st;
+  uint64_t* ht = ctx->host_totals.as<uint64_t>();
+  auto read_totals = [&]() -> int {
+    DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ht, p.totals, 16, cudaMemcpyDeviceToHost, s));
+    DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+    return DPA_OK;
+  };
+  if (!early && (st = read_totals()) != DPA_OK) return st;
   DPA_TRY_CUDA(ctx, ctx->out_vertices.reserve((early ? p.raw_total : ht[0]) * 12));
   DPA_TRY_CUDA(ctx, ctx->out_colors.reserve((early ? p.raw_total : ht[0]) * 4));
   DPA_TRY_CUDA(ctx, ctx->out_indices.reserve(2 * (early ? p.raw_total : ht[1]) * index_bytes));
-  st = emit_curves(ctx, o, n, p, *round_vertices, ctx->out_vertices.as<float>(),
+  st = emit_curves(ctx, o, n, p, scans, *round_vertices, ctx->out_vertices.as<float>(),
                    ctx->out_colors.as<float>(), ctx->out_indices.ptr);
   if (st != DPA_OK) return st;
-  if (early) DPA_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+  if (early && (st = read_totals()) != DPA_OK) return st;
   const uint64_t piece_vertices = ht[0];
   const uint64_t piece_segments = ht[1];
   const uint64_t piece_indices = 2 * piece_segments;
@@ -919,9 +932,11 @@ int dpa_advect_round(dpa_context* ctx, const dpa_field* field, const dpa_advect_
                               s);
       if (st != DPA_OK) return st;
     } else if (whole) {
-      st = advect_curves(ctx, field, options, k, count, p);
+      const bool scans = count > dpa::kEmitScans;
+      st = advect_curves(ctx, field, options, k, count, p, scans);
       if (st == DPA_OK)
-        st = emit_curves(ctx, options, count, p, 0, reinterpret_cast<float*>(device + at.vertices),
+        st = emit_curves(ctx, options, count, p, scans, 0,
+                         reinterpret_cast<float*>(device + at.vertices),
                          reinterpret_cast<float*>(device + at.colors), device + at.indices);
       if (st != DPA_OK) return st;
     } else {

@@ -56,7 +56,16 @@ __device__ __forceinline__ float angular_velocity(const V3& a, const V3& b) {
   return atan2f(norm, dot);
 }
 
-template <bool kIndex64, bool kColors>
+// Sum of counts[0 .. n) over a warp.
+__device__ __forceinline__ uint64_t warp_sum(const uint32_t* counts, uint64_t n, unsigned lane) {
+  uint64_t sum = 0;
+  for (uint64_t i = lane; i < n; i += 32) sum += counts[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  return sum;
+}
+
+template <bool kIndex64, bool kColors, bool kScan>
 __global__ void __launch_bounds__(kEmitWarps * 32) emit_kernel(const EmitArgs e) {
   const uint64_t k = uint64_t(blockIdx.x) * kEmitWarps + (threadIdx.x >> 5);
   if (k >= e.count) return;
@@ -67,7 +76,18 @@ __global__ void __launch_bounds__(kEmitWarps * 32) emit_kernel(const EmitArgs e)
   const float* raw = e.raw_vertices + 3 * e.raw_offsets[k];
   const uint64_t raw_in = e.remaining_in ? e.remaining_in[k] + 2 : e.raw_offsets[k + 1] - e.raw_offsets[k];
   const uint64_t raw_count = raw_in - e.remaining[k];
-  const uint64_t first = e.vertex_offsets[k];
+  uint64_t first, segment;
+  if constexpr (kScan) {
+    first = warp_sum(e.kept_vertices, k, lane);
+    segment = warp_sum(e.kept_segments, k, lane);
+    if (k + 1 == e.count && lane == 0) {
+      e.totals[0] = first + e.kept_vertices[k];
+      e.totals[1] = segment + e.kept_segments[k];
+    }
+  } else {
+    first = e.vertex_offsets[k];
+    segment = e.segment_offsets[k];
+  }
   uint64_t cursor = first;
   for (uint64_t j0 = 0; j0 < raw_count; j0 += 32) {
     const uint64_t j = j0 + lane;
@@ -88,7 +108,6 @@ __global__ void __launch_bounds__(kEmitWarps * 32) emit_kernel(const EmitArgs e)
   // into another particle's curve; the reference's "vertex_index > 1" test
   // (color_generator.cpp:50) is applied to the round-level index.
   const uint64_t kept = e.kept_vertices[k];
-  uint64_t segment = e.segment_offsets[k];
   for (uint64_t m0 = 0; m0 < kept; m0 += 32) {
     const uint64_t m = m0 + lane;
     const bool valid = m < kept;
@@ -341,13 +360,18 @@ inline unsigned blocks_for(uint64_t n, unsigned block) { return unsigned((n + bl
 cudaError_t launch_emit(const EmitArgs& e, bool index64, bool colors, cudaStream_t stream) {
   if (e.count == 0) return cudaSuccess;
   const dim3 grid(blocks_for(e.count, kEmitWarps)), block(kEmitWarps * 32);
-  if (index64) {
-    if (colors) emit_kernel<true, true><<<grid, block, 0, stream>>>(e);
-    else emit_kernel<true, false><<<grid, block, 0, stream>>>(e);
-  } else {
-    if (colors) emit_kernel<false, true><<<grid, block, 0, stream>>>(e);
-    else emit_kernel<false, false><<<grid, block, 0, stream>>>(e);
-  }
+  auto launch = [&](auto scan) {
+    constexpr bool kScan = decltype(scan)::value;
+    if (index64) {
+      if (colors) emit_kernel<true, true, kScan><<<grid, block, 0, stream>>>(e);
+      else emit_kernel<true, false, kScan><<<grid, block, 0, stream>>>(e);
+    } else {
+      if (colors) emit_kernel<false, true, kScan><<<grid, block, 0, stream>>>(e);
+      else emit_kernel<false, false, kScan><<<grid, block, 0, stream>>>(e);
+    }
+  };
+  if (e.vertex_offsets) launch(std::false_type{});
+  else launch(std::true_type{});
   return cudaGetLastError();
 }
 

@@ -148,6 +148,10 @@ struct EmitArgs {
                                   // raw_offsets holds count + 1 entries
   const uint64_t* vertex_offsets; // exclusive scan of kept vertices (piece-local)
   const uint64_t* segment_offsets;// exclusive scan of kept segments (piece-local)
+  // Without the scans (null; at most kEmitScans particles) each particle sums the
+  // counts before its own, and the last writes both totals.
+  unsigned long long* totals;
+  const uint32_t* kept_segments;
   const uint32_t* kept_vertices;
   uint64_t vertex_base;           // round-level index of the piece's first vertex
   float* vertices;                // piece output
@@ -155,6 +159,7 @@ struct EmitArgs {
   void* indices;                  // piece output (uint32 or uint64)
 };
 
+constexpr uint64_t kEmitScans = 1024;
 cudaError_t launch_emit(const EmitArgs& e, bool index64, bool colors, cudaStream_t stream);
 
 // Exclusive scans of the per-particle kept-vertex and kept-segment counts

@@ -16,7 +16,7 @@ def grids():
     return fields.curl_noise(24, 3.0, 3), fields.double_gyre((16, 8, 8), 5)
 
 
-@pytest.mark.parametrize("count", [1, 2, 1184, 1185, 2368, 2369, 4737, 9473, 18944, 18945])
+@pytest.mark.parametrize("count", [1, 2, 1024, 1025, 1184, 1185, 2368, 2369, 4737, 9473, 18944, 18945])
 def test_particles_per_warp(ctx, oracle, grids, count):
     steady, gyre = grids
     rng = np.random.default_rng(count)
