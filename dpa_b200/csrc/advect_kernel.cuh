@@ -59,9 +59,10 @@ constexpr int advect_min_blocks() {
 // kPPT slots of a lane step in lock-step, so one particle's corner gather is
 // in flight while the other's arithmetic issues. An empty slot holds a parked
 // position, the centre of the first cell (never NaN, which would send the
-// division of a step into its slow path for the whole warp). With one
-// particle per lane the branch-free steady Euler and RK4 steppers step a
-// parked slot and discard the result; otherwise an empty slot takes no steps.
+// division of a step into its slow path for the whole warp) at the middle of the
+// first time slice. With one particle per lane the branch-free Euler and RK4
+// steppers step a parked slot and discard the result; otherwise an empty slot
+// takes no steps.
 template <int kIntegrator, int kStorage, int kLocate, bool kRecord, bool kUnsteady, int kPPT>
 __global__ void __launch_bounds__(kAdvectBlock, advect_min_blocks<kIntegrator, kRecord, kUnsteady, kPPT>())
 advect_kernel(const FieldView f, const AdvectArgs a) {
@@ -95,9 +96,10 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
   const Position parked{__fmaf_rn(0.5f, f.spacing[0], f.offset[0]),
                         make_float2(__fmaf_rn(0.5f, f.spacing[2], f.offset[2]),
                                     __fmaf_rn(0.5f, f.spacing[1], f.offset[1]))};
+  const float parked_time = __fmaf_rn(0.5f, f.time_spacing, f.time_origin);
   // (One particle per lane only: with two, skipping a pair's empty slot by a
   // branch measured 1.7x faster on the 512^3 batch than stepping it.)
-  constexpr bool kStepAll = kPPT == 1 && !kUnsteady &&
+  constexpr bool kStepAll = kPPT == 1 &&
                             (kIntegrator == DPA_INTEGRATOR_EULER ||
                              kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4);
 
@@ -113,7 +115,7 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
     active[j] = false;
     p[j] = parked;
     history[j] = StepHistory{};
-    t[j] = 0.0f;
+    t[j] = parked_time;
     curve[j] = nullptr;
   }
 
@@ -292,6 +294,7 @@ advect_kernel(const FieldView f, const AdvectArgs a) {
         atomicSub(a.in_flight + a.request_of[k], 1u);
       active[j] = false;
       p[j] = parked;
+      if constexpr (kUnsteady) t[j] = parked_time;
     }
   }
 }

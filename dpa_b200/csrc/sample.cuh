@@ -426,7 +426,7 @@ struct CellSampler {
   // an outside position loads no corners, and its sample (from the cached
   // ones) is to be discarded.
   __device__ __forceinline__ bool sample_selected(const FieldView& f, const Position& p,
-                                                  float2& v01, float& v2) {
+                                                  float /*t*/, float2& v01, float& v2) {
     Cell c;
     Weights w;
     const bool inside = locate<kLocate>(f, p, c, w);
@@ -443,7 +443,6 @@ struct CellSampler {
     return inside;
   }
 
-  static constexpr bool kSteady = true;
   // (An edge-record field's kernels are at their register limit.)
   static constexpr bool kPackedSums = kStorage != DPA_STORAGE_F32_EDGES;
 
@@ -486,16 +485,18 @@ struct TimeSampler {
   CornersOf<kStorage> lo, hi;  // slices s and s + 1
   uint32_t cached = ~0u, cached_slice = 0;
 
-  __device__ __forceinline__ bool sample(const FieldView& f, const Position& p, float t,
-                                         float2& v01, float& v2) {
+  // Samples at p and time t without an early return, as CellSampler's; outside the
+  // grid or the slices it returns false and loads nothing.
+  __device__ __forceinline__ bool sample_selected(const FieldView& f, const Position& p, float t,
+                                                  float2& v01, float& v2) {
     Cell c;
     Weights w;
-    if (!locate<kLocate>(f, p, c, w)) return false;
-    const CellRows rows = cell_rows<false>(f, c);
     uint32_t slice = 0;
     float wt = 0.0f;
-    if (!locate_time(f, t, slice, wt)) return false;
-    if (rows.at[0] != cached || slice != cached_slice) {
+    const bool here = locate<kLocate>(f, p, c, w);
+    const bool now = locate_time(f, t, slice, wt);
+    const CellRows rows = cell_rows<false>(f, c);
+    if (here && now && (rows.at[0] != cached || slice != cached_slice)) {
       const int64_t base = int64_t(uint64_t(slice) * uint32_t(f.slice_stride));
       gather<kStorage>(f, rows, lo, base);
       gather<kStorage>(f, rows, hi, base + f.slice_stride);
@@ -509,10 +510,14 @@ struct TimeSampler {
     const float u = __fsub_rn(1.0f, wt);
     v01 = blend2(a01, b01, splat(u), splat(wt), make_float2(f.unit[0], f.unit[1]));
     v2 = blend(a2, b2, u, wt);
-    return true;
+    return here && now;
   }
 
-  static constexpr bool kSteady = false;
+  __device__ __forceinline__ bool sample(const FieldView& f, const Position& p, float t,
+                                         float2& v01, float& v2) {
+    return sample_selected(f, p, t, v01, v2);
+  }
+
   static constexpr bool kPackedSums = true;
 
   __device__ __forceinline__ void reset() { cached = ~0u; }
@@ -613,13 +618,13 @@ __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& 
   const float2 unit = make_float2(f.unit[0], f.unit[1]);
   float2 v01;
   float v2;
-  if constexpr (Sampler::kSteady && (kIntegrator == DPA_INTEGRATOR_EULER ||
-                                     kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4)) {
+  if constexpr (kIntegrator == DPA_INTEGRATOR_EULER ||
+                kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4) {
     // Without branches on the outcome: the step is computed whatever the
     // sample, and kept only when the position was inside and the velocity
     // not zero (a step's latency is a dependent chain; the launch's end and
     // launches of few particles wait for it).
-    const bool inside = sampler.sample_selected(f, p, v01, v2);
+    const bool inside = sampler.sample_selected(f, p, t, v01, v2);
     const bool zero = is_zero(v01, v2);
     Position n = p;
     if constexpr (kIntegrator == DPA_INTEGRATOR_EULER) {
