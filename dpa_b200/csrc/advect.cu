@@ -32,11 +32,19 @@ __device__ __forceinline__ uint32_t order_bucket(const FieldView& f, const float
   return (spread6(c[0]) << 2) | (spread6(c[1]) << 1) | spread6(c[2]);
 }
 
-// Bucket ids and their counts. Lanes of a warp that share a bucket (seeds are
-// often dense) add to its counter once.
-__global__ void order_histogram_kernel(const FieldView f, const float* positions, uint64_t count,
-                                       uint32_t* ids, uint32_t* counts, uint32_t resolution,
-                                       uint32_t buckets) {
+// Counters of a tile of the scan over the buckets, and the most tiles.
+constexpr uint32_t kOrderTile = 1024;
+constexpr uint32_t kOrderTiles = (kOrderBuckets + 1 + kOrderTile - 1) / kOrderTile;
+
+// Bucket ids, their counts, and the counts of each tile of buckets: a block adds
+// up its own tiles in shared memory first. Lanes of a warp that share a bucket
+// (seeds are often dense) add to its counter once.
+__global__ void __launch_bounds__(256) order_histogram_kernel(
+    const FieldView f, const float* positions, uint64_t count, uint32_t* ids, uint32_t* counts,
+    uint32_t* tile_sums, uint32_t tiles, uint32_t resolution, uint32_t buckets) {
+  __shared__ uint32_t sums[kOrderTiles];
+  for (uint32_t i = threadIdx.x; i < tiles; i += blockDim.x) sums[i] = 0;
+  __syncthreads();
   for (uint64_t base = uint64_t(blockIdx.x) * blockDim.x; base < count;
        base += uint64_t(gridDim.x) * blockDim.x) {
     const uint64_t t = base + threadIdx.x;
@@ -46,83 +54,53 @@ __global__ void order_histogram_kernel(const FieldView f, const float* positions
     const uint32_t b = order_bucket(f, positions + 3 * t, resolution, buckets);
     ids[t] = b;
     const unsigned same = __match_any_sync(mask, b);
-    if ((threadIdx.x & 31u) == unsigned(__ffs(same) - 1))
+    if ((threadIdx.x & 31u) == unsigned(__ffs(same) - 1)) {
       atomicAdd(&counts[b], uint32_t(__popc(same)));
+      atomicAdd(&sums[b / kOrderTile], uint32_t(__popc(same)));
+    }
   }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < tiles; i += blockDim.x)
+    if (sums[i]) atomicAdd(&tile_sums[i], sums[i]);
 }
 
-// Exclusive scan of the counts in tiles of kScanTile entries: tile sums,
-// a scan of the sums, then each tile's scan plus its prefix. 256 threads,
-// four consecutive entries each.
-constexpr uint32_t kScanTile = 1024;
-
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* warp_sums,
-                                                         uint32_t* total) {
+// Exclusive scan of the counts, a block per tile of kOrderTile (256 threads, four
+// consecutive counters each): its scan after the sums of the tiles before it, which
+// each block adds up itself. Three small launches (tile sums, a scan of them, each
+// tile's scan) took 9.7 us and two gaps for 50,000 seeds, this one 4 (a call that
+// places a 192^3 field and takes ten steps: 124 -> 116 us); launches this small last
+// as long as they take to start.
+__global__ void __launch_bounds__(256) order_scan_kernel(uint32_t* counts, uint32_t n,
+                                                         const uint32_t* tile_sums) {
+  __shared__ uint32_t warp_sums[8], warp_before[8];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+  uint32_t before = 0;
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += 256) before += tile_sums[i];
+  before = __reduce_add_sync(0xffffffffu, before);
+  const uint32_t first = blockIdx.x * kOrderTile + 4 * threadIdx.x;
+  uint32_t v[4], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = first + j < n ? counts[first + j] : 0u;
+    sum += v[j];
+  }
+  uint32_t x = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= unsigned(o)) x += y;
   }
-  if (lane == 31) warp_sums[warp] = x;
+  if (lane == 31) {
+    warp_sums[warp] = x;
+    warp_before[warp] = before;
+  }
   __syncthreads();
-  uint32_t before = 0, all = 0;
-  for (unsigned w = 0; w < blockDim.x / 32; ++w) {
-    if (w < warp) before += warp_sums[w];
-    all += warp_sums[w];
-  }
-  *total = all;
-  return before + x - v;
-}
-
-__device__ __forceinline__ void load_tile(const uint32_t* counts, uint32_t n, uint32_t first,
-                                          uint32_t v[4]) {
+  uint32_t run = x - sum;
+#pragma unroll
+  for (unsigned w = 0; w < 8; ++w) run += warp_before[w] + (w < warp ? warp_sums[w] : 0u);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const uint32_t i = first + 4 * threadIdx.x + j;
-    v[j] = i < n ? counts[i] : 0u;
-  }
-}
-
-__global__ void __launch_bounds__(256) order_tile_sums_kernel(const uint32_t* counts, uint32_t n,
-                                                              uint32_t* tile_sums) {
-  __shared__ uint32_t warp_sums[8];
-  uint32_t v[4];
-  load_tile(counts, n, blockIdx.x * kScanTile, v);
-  uint32_t total = 0;
-  block_exclusive_scan(v[0] + v[1] + v[2] + v[3], warp_sums, &total);
-  if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-// One block: the exclusive scan of up to 256 * 4 tile sums, in place.
-__global__ void __launch_bounds__(256) order_scan_sums_kernel(uint32_t* tile_sums, uint32_t tiles) {
-  __shared__ uint32_t warp_sums[8];
-  uint32_t v[4];
-  load_tile(tile_sums, tiles, 0, v);
-  uint32_t total = 0;
-  uint32_t run = block_exclusive_scan(v[0] + v[1] + v[2] + v[3], warp_sums, &total);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t i = 4 * threadIdx.x + j;
-    if (i < tiles) tile_sums[i] = run;
-    run += v[j];
-  }
-}
-
-__global__ void __launch_bounds__(256) order_scan_tiles_kernel(uint32_t* counts, uint32_t n,
-                                                               const uint32_t* tile_prefix) {
-  __shared__ uint32_t warp_sums[8];
-  uint32_t v[4];
-  const uint32_t first = blockIdx.x * kScanTile;
-  load_tile(counts, n, first, v);
-  uint32_t total = 0;
-  uint32_t run = tile_prefix[blockIdx.x] +
-                 block_exclusive_scan(v[0] + v[1] + v[2] + v[3], warp_sums, &total);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t i = first + 4 * threadIdx.x + j;
-    if (i < n) counts[i] = run;
+    if (first + j < n) counts[first + j] = run;
     run += v[j];
   }
 }
@@ -299,15 +277,13 @@ cudaError_t launch_order(const FieldView& f, const float* positions, uint64_t co
   while (p < resolution) p *= 2;
   const uint32_t buckets = p * p * p;
   const uint32_t n = buckets + 1;  // the last counts the particles outside the grid
-  const uint32_t tiles = (n + kScanTile - 1) / kScanTile;
-  uint32_t* tile_sums = counts + kOrderBuckets + 1;
-  DPA_CUDA_TRY(cudaMemsetAsync(counts, 0, n * sizeof(uint32_t), stream));
+  const uint32_t tiles = (n + kOrderTile - 1) / kOrderTile;
+  uint32_t* tile_sums = counts + n;
+  DPA_CUDA_TRY(cudaMemsetAsync(counts, 0, (n + tiles) * sizeof(uint32_t), stream));
   const uint64_t blocks = std::min<uint64_t>((count + 255) / 256, 4 * 148);
-  order_histogram_kernel<<<unsigned(blocks), 256, 0, stream>>>(f, positions, count, ids, counts,
-                                                               resolution, buckets);
-  order_tile_sums_kernel<<<tiles, 256, 0, stream>>>(counts, n, tile_sums);
-  order_scan_sums_kernel<<<1, 256, 0, stream>>>(tile_sums, tiles);
-  order_scan_tiles_kernel<<<tiles, 256, 0, stream>>>(counts, n, tile_sums);
+  order_histogram_kernel<<<unsigned(blocks), 256, 0, stream>>>(
+      f, positions, count, ids, counts, tile_sums, tiles, resolution, buckets);
+  order_scan_kernel<<<tiles, 256, 0, stream>>>(counts, n, tile_sums);
   order_scatter_kernel<<<unsigned((count + 255) / 256), 256, 0, stream>>>(ids, count, counts,
                                                                            order);
   return cudaGetLastError();

@@ -114,7 +114,7 @@ cudaError_t prepare_advect(const FieldView& f, const AdvectArgs& a, int integrat
 
 // Processing order: a counting sort of the particles by the Morton code of
 // their start cell on a resolution^3 coarsening of the grid (a memset and
-// five kernels). Within a bucket the order is arbitrary; results never depend
+// three kernels). Within a bucket the order is arbitrary; results never depend
 // on processing order. ids holds count bucket ids; counts holds
 // kOrderCountsSize counters (the buckets of the finest resolution, one for
 // particles outside the grid, and the scan's tile sums).
@@ -122,9 +122,9 @@ constexpr uint32_t kOrderMaxResolution = 64;
 constexpr uint32_t kOrderDefaultResolution = 64;
 constexpr uint32_t kOrderBuckets = kOrderMaxResolution * kOrderMaxResolution * kOrderMaxResolution;
 constexpr uint32_t kOrderCountsSize = kOrderBuckets + 1 + (kOrderBuckets + 1 + 1023) / 1024;
-constexpr int kOrderLaunches = 5;
+constexpr int kOrderLaunches = 3;
 // Calls with fewer particles run in input order: their warps share few cells,
-// and the sort's six launches cost more than the locality gains (4096 seeds of
+// and the sort's launches cost more than the locality gains (4096 seeds of
 // the recording configuration: 0.90 ms per round unsorted, 0.94 sorted).
 constexpr uint64_t kOrderMinParticles = 8192;
 
