@@ -42,6 +42,27 @@ constexpr int advect_min_blocks() {
                                                          : kAdvectMinBlocks;
 }
 
+// Pathlines of F32 nodes by Euler and RK4 also come as narrow kernels (kNarrowBit
+// of the mode): held to 96 registers, with four words spilled around the gather, and
+// launched in blocks of 64, which gives each of an SM's register files 5 warps
+// instead of 4. Issue was busy 57 % of the time at 4. 250,000 pathlines of 1000 steps
+// 3054 -> 2654 us, from edge records 2930 -> 2685; F16 fields, issue-bound at 67 to
+// 72 %, gain nothing (2926 -> 3007), the four-sample stepper spills (2863 -> 2943).
+template <int kIntegrator, int kStorage, bool kRecord, bool kUnsteady>
+constexpr bool advect_has_narrow() {
+  return kUnsteady && !kRecord &&
+         (kStorage == DPA_STORAGE_F32 || kStorage == DPA_STORAGE_F32_EDGES) &&
+         (kIntegrator == DPA_INTEGRATOR_EULER || kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4);
+}
+
+// Registers per thread: what the block count leaves (allocated by eights).
+template <int kIntegrator, int kLocate, bool kRecord, bool kUnsteady, int kPPT>
+constexpr int advect_registers() {
+  return kLocate & kNarrowBit
+             ? 96
+             : 65536 / (kAdvectBlock * advect_min_blocks<kIntegrator, kRecord, kUnsteady, kPPT>()) / 8 * 8;
+}
+
 // Persistent advection. Every lane owns kPPT slots, each holding one particle
 // at a time; a slot whose particle finishes takes the next one from its
 // warp's claim of a.claim consecutive entries of the processing order, and
@@ -64,9 +85,9 @@ constexpr int advect_min_blocks() {
 // steppers step a parked slot and discard the result; otherwise an empty slot
 // takes no steps.
 template <int kIntegrator, int kStorage, int kLocate, bool kRecord, bool kUnsteady, int kPPT>
-__global__ void __launch_bounds__(kAdvectBlock, advect_min_blocks<kIntegrator, kRecord, kUnsteady, kPPT>())
+__global__ void __maxnreg__((advect_registers<kIntegrator, kLocate, kRecord, kUnsteady, kPPT>()))
 advect_kernel(const FieldView f, const AdvectArgs a) {
-  using Sampler = std::conditional_t<kUnsteady, TimeSampler<kStorage, kLocate>,
+  using Sampler = std::conditional_t<kUnsteady, TimeSampler<kStorage, kLocate & ~kNarrowBit>,
                                      CellSampler<kStorage, kLocate>>;
   constexpr unsigned kFull = 0xffffffffu;
   // State touched only when particles are handed out or finish lives in
@@ -323,15 +344,15 @@ cudaError_t resident_blocks(uint32_t block, int* blocks_per_sm, int* sms) {
   return cudaSuccess;
 }
 
-// Threads per block of a launch: the tuning's choice, else kAdvectBlock, or
+// Threads per block of a launch: the tuning's choice, else the kernel's own, or
 // fewer (a multiple of 32) when the particles would fill fewer blocks than
 // the device has SMs, so that a small launch still spreads over every SM.
-inline uint32_t advect_block(const AdvectArgs& a, uint64_t lanes, int sms) {
+inline uint32_t advect_block(const AdvectArgs& a, uint32_t own, uint64_t lanes, int sms) {
   if (a.block) return a.block;
-  uint32_t block = uint32_t(kAdvectBlock);
+  uint32_t block = own;
 #if DPA_ADVECT_SPREAD
   const uint64_t per_sm = (lanes + uint64_t(sms) - 1) / uint64_t(sms);
-  if (per_sm < uint64_t(kAdvectBlock)) block = uint32_t(std::max<uint64_t>(32, (per_sm + 31) / 32 * 32));
+  if (per_sm < uint64_t(own)) block = uint32_t(std::max<uint64_t>(32, (per_sm + 31) / 32 * 32));
 #else
   (void)lanes;
   (void)sms;
@@ -362,7 +383,7 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
       kAdvectBlock, &resident, &sms)));
   const bool free_shape = kPPT == 1 && !a.block && !a.blocks_per_sm;
   const uint32_t own = free_shape ? particles_per_warp(a.count, sms) : 32u * kPPT;
-  const uint32_t block = own < 32 ? 32 : advect_block(a, lanes, sms);
+  const uint32_t block = own < 32 ? 32 : advect_block(a, kLocate & kNarrowBit ? 64 : kAdvectBlock, lanes, sms);
   if (block == 0 || block % 32 != 0 || block > uint32_t(kAdvectBlock)) return cudaErrorInvalidValue;
   DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>(
       block, &resident, &sms)));
@@ -392,6 +413,21 @@ cudaError_t launch_ppt(const FieldView& f, const AdvectArgs& a, cudaStream_t s) 
   if constexpr (!kRecord && !kUnsteady && kIntegrator != DPA_INTEGRATOR_RUNGE_KUTTA_4_TRUE) {
     if (a.particles_per_thread == 2)
       return launch_typed<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, 2>(f, a, s);
+  }
+  if constexpr (advect_has_narrow<kIntegrator, kStorage, kRecord, kUnsteady>()) {
+    // Narrow where the wide kernel cannot hold every particle at once; where it can,
+    // a launch lasts as long as its longest chain of steps, and the spills lengthen
+    // that (8000 pathlines 600 -> 608 us). A tuning's launch shape is the wide
+    // kernel's. A launch of nothing prepares both.
+    int sms = 0, resident = 0;
+    DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, 1>(
+        kAdvectBlock, &resident, &sms)));
+    const uint64_t held = uint64_t(resident) * uint64_t(sms) * kAdvectBlock;
+    if (a.count == 0 || (a.count > held && !a.block && !a.blocks_per_sm)) {
+      const cudaError_t e =
+          launch_typed<kIntegrator, kStorage, kLocate | kNarrowBit, kRecord, kUnsteady, 1>(f, a, s);
+      if (a.count != 0 || e != cudaSuccess) return e;
+    }
   }
   return launch_typed<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, 1>(f, a, s);
 }

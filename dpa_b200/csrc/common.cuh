@@ -37,6 +37,8 @@ enum LocateMode : int { kLocateDivide = 0, kLocateReciprocal = 1, kLocatePow2 = 
 
 // Kernels of a tiled field are instantiated with this bit beside the mode.
 constexpr int kTiledBit = 4;
+// And the narrow ones of a time-varying field with this one (advect_kernel.cuh).
+constexpr int kNarrowBit = 8;
 
 // Node layout of large steady fields: tiles of about one 2 MiB page instead of
 // rows, so that the particles of an SM stay in few pages. Node (i0, i1, i2) of a
