@@ -92,17 +92,22 @@ __device__ __noinline__ double max_eigenvalue_jacobi(double a[3][3]) {
 // r = det(B) / (2 p^3), the eigenvalues are q + p x for the roots x of
 // x^3 - 3 x = 2 r. For r >= 0 the largest root lies apart, in [sqrt 3, 2], where
 // the cubic's slope is at least 6. It is found by Newton steps, two in 32 bits
-// from the chord of [sqrt 3, 2] (1e-7) and two in 64 with the 32-bit slope, which
+// from the chord of [sqrt 3, 2] (1e-7) and two in 64 with the 32-bit slope there, which
 // leave rounding errors only. For r < 0 that root is the smallest eigenvalue's, with
 // its sign changed, and the largest is -x / 2 away from it plus half the gap of
-// the other two, sqrt(3 - 3/4 x^2). The gap loses digits as it closes:
-// 1 + r = 1e-8 leaves a relative error of 4e-12 in the eigenvalue, far below the
-// 6e-8 of the 32-bit result. Closer than that (a double largest eigenvalue) and
-// for matrices that are not finite it returns false: the Jacobi rotations answer.
+// the other two, sqrt(3 - 3/4 x^2). The gap loses digits as it closes: the rounding of
+// q alone, 2^-53 q, moves the eigenvalue by 2^-54 q / gap. The FTLE is the logarithm,
+// which is nearly |1 - largest| where that is small (a flow map near the identity), so
+// cells with gap * |1 - largest| below 2^-16 (1 + q) return false, as matrices that are
+// not finite do, and the Jacobi rotations answer. What is left is a relative error of
+// 1e-11 in the logarithm, beside what the rotations have too (random matrices I + s S, s
+// from 1e-6 to 1, the two largest eigenvalues 1e-4 to 1 of s apart, against 80 bits),
+// where the 32-bit result has 6e-8.
 //
 // The rotations throughout took 1900 warp instructions for 32 cells, 800 of them in
 // 64 bits: 132 us for 1.5 million cells at 70 % of the issue slots; this took 480
-// and 32 us, and 430 and 27 us with the divisions of cauchy_green().
+// and 32 us, and 430 and 27 us with the divisions of cauchy_green(). In a stream of
+// calls that is 21.8 us, and 22.8 with the test of the gap.
 __device__ __forceinline__ bool max_eigenvalue(const double a[3][3], double& largest) {
   const double q = (a[0][0] + a[1][1] + a[2][2]) * (1.0 / 3.0);
   const double b0 = a[0][0] - q, b1 = a[1][1] - q, b2 = a[2][2] - q;
@@ -114,22 +119,26 @@ __device__ __forceinline__ bool max_eigenvalue(const double a[3][3], double& lar
   const double half_det =
       0.5 * (b0 * (b1 * b2 - w * w) - u * (u * b2 - w * v) + v * (u * w - b1 * v));
   const double r = half_det * inverse * inverse * inverse;
-  if (!(r >= -1.0 + 1e-8) || !(p2 < 1e300)) return false;
+  if (!(p2 < 1e300)) return false;
   const double two_r = fmin(2.0 * fabs(r), 2.0);
   constexpr float kRoot3 = 1.7320508f;
   float x0 = fmaf(0.5f * (2.0f - kRoot3), float(two_r), kRoot3);
-  float slope = 0.0f;
+  float slope = __fdividef(1.0f, fmaf(3.0f * x0, x0, -3.0f));
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    slope = __fdividef(1.0f, fmaf(3.0f * x0, x0, -3.0f));
     x0 -= fmaf(fmaf(x0, x0, -3.0f), x0, -float(two_r)) * slope;
+    slope = __fdividef(1.0f, fmaf(3.0f * x0, x0, -3.0f));
   }
   double x = x0;
 #pragma unroll
   for (int i = 0; i < 2; ++i) x -= fma(fma(x, x, -3.0), x, -two_r) * double(slope);
-  if (r < 0.0) x = 0.5 * x + sqrt(fmax(fma(-0.75 * x, x, 3.0), 0.0));
+  double gap = 2.0;
+  if (r < 0.0) {
+    gap = sqrt(fmax(fma(-0.75 * x, x, 3.0), 0.0));
+    x = 0.5 * x + gap;
+  }
   largest = fma(p, x, q);
-  return true;
+  return r >= 0.0 || gap * fabs(largest - 1.0) >= fma(0x1p-16, q, 0x1p-16);
 }
 
 // C = J^T J of a lattice cell in FP32 (Eigen's 3x3 lazy product, c0 + (c1 + c2)),
