@@ -1202,7 +1202,19 @@ int dpa_ftle_estimate_device(dpa_context* ctx, const dpa_field* field, const flo
     a.final_positions = device_final_positions;
     a.winners = ctx->ftle_winners.ptr;
     a.ftle = device_ftle;
+    // Cells read their neighbours' final positions: a result that takes the place of
+    // the positions goes through the context's own array.
+    const auto at = [](const void* x) { return reinterpret_cast<uintptr_t>(x); };
+    const bool in_place = at(device_ftle) < at(device_final_positions) + count * 12 &&
+                          at(device_final_positions) < at(device_ftle) + cells * 4;
+    if (in_place) {
+      DPA_TRY_CUDA(ctx, ctx->ftle_out.reserve(cells * 4));
+      a.ftle = ctx->ftle_out.as<float>();
+    }
     DPA_TRY_CUDA(ctx, dpa::launch_ftle(a, s));
+    if (in_place)
+      DPA_TRY_CUDA(ctx, cudaMemcpyAsync(device_ftle, a.ftle, cells * 4, cudaMemcpyDeviceToDevice,
+                                        s));
     return DPA_OK;
   });
 }
