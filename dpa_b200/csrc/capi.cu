@@ -107,6 +107,7 @@ int advect_device_impl(dpa_context* ctx, const dpa_field* field, const dpa_advec
     if (st != DPA_OK) return st;
   }
   if (count == 0) return DPA_OK;
+  DPA_TRY_CUDA(ctx, dpa::note_stream(ctx, field, s));
   dpa_launch_scratch& scratch = own_scratch ? *own_scratch : ctx->scratch;
   if (ctx->profiling) DPA_TRY_CUDA(ctx, cudaEventRecord(ctx->events[0], s));
   const uint32_t* order = nullptr;
@@ -837,8 +838,10 @@ int dpa_field_destroy(dpa_context* ctx, dpa_field* field) {
   if (!ctx || !field) return DPA_ERROR_INVALID_ARGUMENT;
   if (field->owner != ctx) return fail(ctx, DPA_ERROR_INVALID_ARGUMENT, "field belongs to another context");
   cudaSetDevice(ctx->device);
-  // Calls on any stream may still read the field; its block may be the next one's.
-  if (cudaDeviceSynchronize() == cudaSuccess) field->nodes.release_to(ctx->spare);
+  // Once the context's stream has finished, the block of a field used only there may be
+  // the next one's.
+  if (cudaStreamSynchronize(ctx->stream) == cudaSuccess && !field->elsewhere)
+    field->nodes.release_to(ctx->spare);
   field->nodes.release();
   delete field;
   return DPA_OK;

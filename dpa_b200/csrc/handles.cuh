@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -255,5 +256,21 @@ struct dpa_field {
   uint32_t slices = 1;  // > 1: a time-varying field
   float time_origin = 0.0f;
   float time_spacing = 0.0f;
+  // Whether work elsewhere than in the context's stream may read the nodes: a caller's
+  // stream, a graph or a server. Such a field's block is freed, not kept: only cudaFree
+  // waits for that work without a device-wide wait, which CUDA forbids while any thread
+  // captures a stream of the device.
+  mutable std::atomic<bool> elsewhere{false};
 };
+
+namespace dpa {
+// Notes that work reading the field's nodes goes to stream s.
+inline cudaError_t note_stream(const dpa_context* ctx, const dpa_field* field, cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (s == ctx->stream) DPA_CUDA_TRY(cudaStreamIsCapturing(s, &status));
+  if (s != ctx->stream || status != cudaStreamCaptureStatusNone)
+    field->elsewhere.store(true, std::memory_order_relaxed);
+  return cudaSuccess;
+}
+}  // namespace dpa
 

@@ -89,6 +89,8 @@ extern "C" int dpa_advect_device_no_alloc(dpa_context* ctx, const dpa_field* fie
     e = scratch_on(ctx->device, &scratch);
     if (e != cudaSuccess) return dpa::fail_cuda(ctx, e, "cudaGetSymbolAddress");
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+    e = dpa::note_stream(ctx, field, s);
+    if (e != cudaSuccess) return dpa::fail_cuda(ctx, e, "cudaStreamIsCapturing");
 
     // The context's tuning applies as it does to dpa_advect_device: launch
     // shape, claims and processing order (resolution, or input order when 0).

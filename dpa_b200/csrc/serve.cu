@@ -804,6 +804,7 @@ int dpa_server_add_field(dpa_server* s, const dpa_field* field, int32_t* id) {
     return DPA_ERROR_INVALID_ARGUMENT;
   }
   s->fields.push_back(field);
+  field->elsewhere = true;
   *id = int32_t(s->fields.size() - 1);
   return DPA_OK;
 }
