@@ -177,6 +177,7 @@ SIGNATURES = {
     "dpa_context_synchronize": (C.c_int, [_P]),
     "dpa_context_set_staging_limit": (C.c_int, [_P, C.c_uint64]),
     "dpa_context_set_host_chunk_limit": (C.c_int, [_P, C.c_uint64]),
+    "dpa_context_set_spare_limit": (C.c_int, [_P, C.c_uint64]),
     "dpa_context_set_profiling": (C.c_int, [_P, C.c_int32]),
     "dpa_context_last_timing": (C.c_int, [_P, _F32P, _F32P]),
     "dpa_context_last_emit_timing": (C.c_int, [_P, _F32P]),

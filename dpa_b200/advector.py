@@ -160,6 +160,9 @@ class Context:
     def set_staging_limit(self, nbytes: int) -> None:
         self.check(self._lib.dpa_context_set_staging_limit(self.handle, int(nbytes)))
 
+    def set_spare_limit(self, nbytes: int) -> None:
+        self.check(self._lib.dpa_context_set_spare_limit(self.handle, int(nbytes)))
+
     def field(self, grid: RegularGrid, storage: str = "f32") -> "Field":
         return Field(self, grid, storage)
 

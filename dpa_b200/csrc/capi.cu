@@ -507,6 +507,13 @@ int dpa_context_set_host_chunk_limit(dpa_context* ctx, uint64_t bytes) {
   return DPA_OK;
 }
 
+int dpa_context_set_spare_limit(dpa_context* ctx, uint64_t bytes) {
+  if (!ctx) return DPA_ERROR_INVALID_ARGUMENT;
+  DPA_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
+  ctx->spare.set_limit(size_t(bytes));
+  return DPA_OK;
+}
+
 int dpa_context_set_profiling(dpa_context* ctx, int32_t enabled) {
   if (!ctx) return DPA_ERROR_INVALID_ARGUMENT;
   DPA_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
@@ -703,11 +710,12 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     for (int i = 0; i < 3; ++i) f->view.n[i] = int32_t(shape[i]);
     f->view.storage = storage;
     f->node_bytes = std::max<uint64_t>(dpa::choose_layout(f->view, slices) * node_bytes, 16);
-    cudaError_t e = f->nodes.reserve_from(ctx->spare, f->node_bytes);
+    bool kept = false, copy_kept = false;
+    cudaError_t e = f->nodes.reserve_from(ctx->spare, f->node_bytes, &kept);
     const float* src = xyzv;
     DeviceBuffer staging;
     if (e == cudaSuccess && !device_input) {
-      e = staging.reserve_from(ctx->spare, nodes * 12);
+      e = staging.reserve_from(ctx->spare, nodes * 12, &copy_kept);
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(staging.ptr, xyzv, nodes * 12, cudaMemcpyHostToDevice, ctx->stream);
       src = staging.as<float>();
@@ -715,7 +723,8 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     if (e == cudaSuccess)
       e = dpa::launch_repack(src, nodes, f->view, f->nodes.ptr, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess) staging.release_to(ctx->spare);
+    // A program that makes fields over and over again needs the copy's block again too.
+    if (e == cudaSuccess && (kept || copy_kept)) staging.release_to(ctx->spare);
     staging.release();
     if (e != cudaSuccess) {
       f->nodes.release();

@@ -14,13 +14,13 @@ namespace dpa {
 
 // Device blocks of destroyed fields, kept for the next field of about their size:
 // a program that makes a field of each time step would otherwise spend more on
-// allocating and freeing it than on using it. At most kKeep bytes in kMost blocks
-// stay; the oldest go first, all when the context goes or when an allocation of any
-// context of the process finds no memory. Blocks are given back only when the device
-// has finished with them.
+// allocating and freeing it than on using it. At most limit_ bytes in kMost blocks
+// stay (a larger block is freed at once); the oldest go first, all when the context goes
+// or when an allocation of any context of the process finds no memory. Blocks are given
+// back only when the device has finished with them.
 class SpareBlocks {
  public:
-  static constexpr size_t kKeep = size_t(1) << 30, kMost = 4;
+  static constexpr size_t kMost = 4;
   SpareBlocks() {
     std::lock_guard<std::mutex> guard(registry().lock);
     registry().all.push_back(this);
@@ -37,30 +37,30 @@ class SpareBlocks {
   // A kept block of n bytes or up to an eighth more, or null.
   void* take(size_t n, size_t* bytes) {
     std::lock_guard<std::mutex> guard(lock_);
-    for (size_t i = 0; i < blocks_.size(); ++i) {
+    for (size_t i = 0; i < count_; ++i) {
       if (blocks_[i].bytes < n || blocks_[i].bytes - n > n / 8) continue;
-      void* ptr = blocks_[i].ptr;
       *bytes = blocks_[i].bytes;
-      blocks_.erase(blocks_.begin() + long(i));
-      return ptr;
+      return remove(i);
     }
     return nullptr;
   }
   void give(void* ptr, size_t bytes) {
     std::lock_guard<std::mutex> guard(lock_);
-    blocks_.push_back({ptr, bytes});
-    size_t held = 0;
-    for (const block& b : blocks_) held += b.bytes;
-    while (!blocks_.empty() && (held > kKeep || blocks_.size() > kMost)) {
-      held -= blocks_.front().bytes;
-      cudaFree(blocks_.front().ptr);
-      blocks_.erase(blocks_.begin());
+    if (bytes > limit_) {
+      cudaFree(ptr);
+      return;
     }
+    shrink(limit_ - bytes, kMost - 1);
+    blocks_[count_++] = {ptr, bytes};
   }
   void release() {
     std::lock_guard<std::mutex> guard(lock_);
-    for (const block& b : blocks_) cudaFree(b.ptr);
-    blocks_.clear();
+    shrink(0, 0);
+  }
+  void set_limit(size_t bytes) {
+    std::lock_guard<std::mutex> guard(lock_);
+    limit_ = bytes;
+    shrink(bytes, kMost);
   }
   // Returns what every context of the process keeps.
   static void release_everywhere() {
@@ -81,8 +81,25 @@ class SpareBlocks {
     static registry_type* r = new registry_type;  // outlives every context
     return *r;
   }
+  void* remove(size_t i) {
+    void* ptr = blocks_[i].ptr;
+    std::copy(blocks_ + i + 1, blocks_ + count_, blocks_ + i);
+    --count_;
+    return ptr;
+  }
+  // Frees the oldest until at most this many bytes and blocks are left.
+  void shrink(size_t bytes, size_t blocks) {
+    size_t held = 0;
+    for (size_t i = 0; i < count_; ++i) held += blocks_[i].bytes;
+    while (count_ && (held > bytes || count_ > blocks)) {
+      held -= blocks_[0].bytes;
+      cudaFree(remove(0));
+    }
+  }
   std::mutex lock_;
-  std::vector<block> blocks_;
+  size_t limit_ = size_t(1) << 30;
+  block blocks_[kMost];
+  size_t count_ = 0;
 };
 
 // Grow-only device buffer; freed by release() or when it goes out of scope
@@ -112,9 +129,10 @@ struct DeviceBuffer {
     return cudaSuccess;
   }
   // reserve() from the spare blocks where one fits, and release() to them.
-  cudaError_t reserve_from(SpareBlocks& spare, size_t n) {
+  cudaError_t reserve_from(SpareBlocks& spare, size_t n, bool* kept = nullptr) {
     release();
     if (n) ptr = spare.take(n, &bytes);
+    if (kept) *kept = ptr != nullptr;
     return ptr ? cudaSuccess : reserve(n);
   }
   void release_to(SpareBlocks& spare) {

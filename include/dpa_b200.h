@@ -166,6 +166,13 @@ int dpa_context_set_staging_limit(dpa_context* ctx, uint64_t bytes);
  * (1 to 16 MiB of vertices and colors). */
 int dpa_context_set_host_chunk_limit(dpa_context* ctx, uint64_t bytes);
 
+/* Upper bound on the device memory of destroyed fields that the context keeps for
+ * the fields made after them (default 1 GiB, in at most 4 blocks). Other allocators
+ * of the process cannot have that memory: 0 keeps none. What is above the bound is
+ * freed before the call returns, what is kept when the context is destroyed or when
+ * an allocation of this library finds no memory. */
+int dpa_context_set_spare_limit(dpa_context* ctx, uint64_t bytes);
+
 /* Instrumentation, the counterpart of the reference's per-round timers
  * (pipeline.cpp:98-145, benchmark.hpp:152-158). With profiling on, every
  * advection records CUDA events on its stream around the ordering kernels
@@ -217,7 +224,9 @@ int dpa_field_create_device(dpa_context* ctx, const float* device_xyzv, const ui
 
 /* Waits for the context's stream, then frees the field. Graphs captured on a
  * field and servers it was added to keep its device address: destroy them
- * first. */
+ * first. The memory of a field that was used in the context's stream alone is kept
+ * for the next field of about its size (dpa_context_set_spare_limit), with that of
+ * the upload's copy once fields are made of kept memory; any other is freed. */
 int dpa_field_destroy(dpa_context* ctx, dpa_field* field);
 
 int dpa_field_info(const dpa_field* field, uint64_t shape[3], float offset[3], float spacing[3],
