@@ -709,15 +709,21 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     const size_t node_bytes = dpa::field_node_bytes(storage);
     for (int i = 0; i < 3; ++i) f->view.n[i] = int32_t(shape[i]);
     f->view.storage = storage;
-    f->node_bytes = std::max<uint64_t>(dpa::choose_layout(f->view, slices) * node_bytes, 16);
     bool kept = false, copy_kept = false;
-    cudaError_t e = f->nodes.reserve_from(ctx->spare, f->node_bytes, &kept);
-    const float* src = xyzv;
+    cudaError_t e = cudaSuccess;
     DeviceBuffer staging;
+    for (bool rows : {false, true}) {
+      f->node_bytes =
+          std::max<uint64_t>(dpa::choose_layout(f->view, slices, rows) * node_bytes, 16);
+      e = f->nodes.reserve_from(ctx->spare, f->node_bytes, &kept);
+      if (e == cudaSuccess && !device_input)
+        e = staging.reserve_from(ctx->spare, nodes * 12, &copy_kept);
+      // Tiles take a little more memory than rows.
+      if (e != cudaErrorMemoryAllocation || !f->view.tiled) break;
+    }
+    const float* src = xyzv;
     if (e == cudaSuccess && !device_input) {
-      e = staging.reserve_from(ctx->spare, nodes * 12, &copy_kept);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(staging.ptr, xyzv, nodes * 12, cudaMemcpyHostToDevice, ctx->stream);
+      e = cudaMemcpyAsync(staging.ptr, xyzv, nodes * 12, cudaMemcpyHostToDevice, ctx->stream);
       src = staging.as<float>();
     }
     if (e == cudaSuccess)

@@ -45,8 +45,9 @@ constexpr int kNarrowBit = 8;
 // slice is at
 //   sum over axes of i * stride + (i / size) * jump   (stride 1 along axis 2),
 // the quotient i / size being the high word of i * magic (i < 2^23, size <= 64).
-// A tile's rows of nodes hold one node more than the tile, the next tile's first,
-// so that a cell's two nodes along axis 2 always follow each other.
+// Where axis 2 has several tiles, a tile's rows of nodes hold one node more than the
+// tile, the next tile's first, so that a cell's two nodes along it always follow each
+// other.
 struct TileLayout {
   uint32_t magic[3];
   uint32_t stride[2];

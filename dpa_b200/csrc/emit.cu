@@ -431,7 +431,7 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& f,
 // translation cache: random 16-byte gathers fall from 2079 GB/s in a table of
 // 256 MB to 892 in one of 2 GB. Tiles keep a particle's path in fewer pages, and
 // fewer warps in flight leave room for their misses.
-uint64_t choose_layout(FieldView& v, uint32_t slices) {
+uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
   constexpr uint64_t kTileBytes = 512ull << 20, kFewerThreadsBytes = 1280ull << 20;
   const uint64_t node_bytes = field_node_bytes(v.storage);
   const uint64_t nodes = uint64_t(v.n[0]) * uint64_t(v.n[1]) * uint64_t(v.n[2]);
@@ -440,8 +440,10 @@ uint64_t choose_layout(FieldView& v, uint32_t slices) {
   v.threads_per_sm = 0;
   if (slices != 1 || nodes * node_bytes < kTileBytes) return nodes * slices;
   // About 64 nodes an axis, of a 2 MiB page for F32 nodes (axis 2: 32); tiles of
-  // one axis are as even as they can be, so that little is allocated beyond the
-  // field.
+  // one axis are as even as they can be, and a row of one tile ends in no node of the
+  // next, so that at most an eighth is allocated beyond the field (a field of
+  // 65 x 15,645 x 33 F32 nodes 11 %, 512^3 3 %). A field that finds no room for that
+  // lies in rows.
   const bool edges = v.storage == DPA_STORAGE_F32_EDGES;
   const uint32_t want[3] = {64u, edges ? 32u : 64u, v.storage == DPA_STORAGE_F32 || edges ? 32u : 64u};
   uint64_t size[3], tiles[3];
@@ -449,12 +451,12 @@ uint64_t choose_layout(FieldView& v, uint32_t slices) {
     tiles[i] = (uint64_t(v.n[i]) + want[i] - 1) / want[i];
     size[i] = (uint64_t(v.n[i]) + tiles[i] - 1) / tiles[i];
   }
-  const uint64_t row = size[2] + (edges ? 0 : 1);
+  const uint64_t row = size[2] + (edges || tiles[2] == 1 ? 0 : 1);
   const uint64_t tile = size[0] * size[1] * row;
   const uint64_t total = tile * tiles[0] * tiles[1] * tiles[2];
   v.threads_per_sm = 512;
   // An axis of one node would need a magic of 2^32; the index is 32 bits wide.
-  if (size[0] < 2 || size[1] < 2 || size[2] < 2 || total >= (1ull << 32)) return nodes;
+  if (rows || size[0] < 2 || size[1] < 2 || size[2] < 2 || total >= (1ull << 32)) return nodes;
   v.threads_per_sm = total * node_bytes > kFewerThreadsBytes ? 768 : 0;
   v.tiled = 1;
   for (int i = 0; i < 3; ++i) v.tile.magic[i] = uint32_t((1ull << 32) / size[i] + 1);

@@ -122,6 +122,7 @@ struct DeviceBuffer {
       e = cudaMalloc(&ptr, n);
     }
     if (e != cudaSuccess) {
+      cudaGetLastError();  // not the next launch's error
       ptr = nullptr;
       return e;
     }

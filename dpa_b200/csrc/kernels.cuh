@@ -192,10 +192,10 @@ uint64_t field_node_bytes(int storage);
 cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& view, void* out,
                           cudaStream_t stream);
 
-// The layout of a steady field of this shape and storage. Returns the nodes to
-// allocate; sets view.tiled, view.tile and view.threads_per_sm (view.n and
+// The layout of a steady field of this shape and storage, or of its rows. Returns the
+// nodes to allocate; sets view.tiled, view.tile and view.threads_per_sm (view.n and
 // view.storage are set).
-uint64_t choose_layout(FieldView& view, uint32_t slices);
+uint64_t choose_layout(FieldView& view, uint32_t slices, bool rows);
 
 struct FtleArgs {
   uint64_t count;
