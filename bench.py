@@ -286,8 +286,9 @@ def within_horizon(err, bar=0.99):
     return best
 
 
-KERNEL_SOURCES = ["advect_kernel.cuh", "sample.cuh", "common.cuh", "kernels.cuh", "advect.cu",
-                  "advect_f32.cu", "advect_f32e.cu", "advect_f16.cu", "advect_bf16.cu"]
+KERNEL_SOURCES = ["advect_kernel.cuh", "sample.cuh", "common.cuh", "kernels.cuh",
+                  "launch_shape.hpp", "advect.cu", "advect_f32.cu", "advect_f32e.cu",
+                  "advect_f16.cu", "advect_bf16.cu"]
 
 
 def _code_lines(text):

@@ -344,46 +344,6 @@ cudaError_t resident_blocks(uint32_t block, int* blocks_per_sm, int* sms) {
   return cudaSuccess;
 }
 
-// Threads per block of a launch: the tuning's choice, else the kernel's own, or
-// fewer (a multiple of 32) when the particles would fill fewer blocks than
-// the device has SMs, so that a small launch still spreads over every SM. A launch
-// whose blocks all fit at once (resident of them to an SM) but would leave the
-// fullest SM more than a quarter above the average takes blocks of 64: 50,000 seeds
-// are 196 blocks of 256, two on 48 SMs and one on the others. us at 256 and 64:
-// 47,172 seeds of the four-sample stepper, F16, 612 -> 520; 50,000 F16 258 -> 237, F32
-// in 96^3 284 -> 226; 60,000 pathlines 1010 -> 951. More even ones gain little or lose
-// a percent (100,000 F16 seeds, 391 blocks: 329 -> 335).
-inline uint32_t advect_block(const AdvectArgs& a, uint32_t own, uint64_t lanes, int sms,
-                             int resident) {
-  if (a.block) return a.block;
-  uint32_t block = own;
-#if DPA_ADVECT_SPREAD
-  const uint64_t per_sm = (lanes + uint64_t(sms) - 1) / uint64_t(sms);
-  if (per_sm < uint64_t(own)) block = uint32_t(std::max<uint64_t>(32, (per_sm + 31) / 32 * 32));
-  const uint64_t blocks = (lanes + own - 1) / own, n = uint64_t(sms);
-  if (blocks > n && blocks <= uint64_t(resident) * n && 4 * n * ((blocks + n - 1) / n) > 5 * blocks)
-    block = std::min(block, 64u);
-#else
-  (void)lanes;
-  (void)sms;
-  (void)resident;
-#endif
-  return block;
-}
-
-// Particles per warp of a small launch: as few as keep every SM at 8 warps or
-// less (1, 2, 4, 8, 16; else 32). A warp waits at every step for the slowest of its
-// lanes' gathers, and such a launch leaves the SMs' issue slots idle; more warps per
-// SM than that take turns instead. B200, us at 32 lanes and as chosen: 100 recorded
-// seeds 33 -> 21 (1 lane), 1000 216 -> 168 (1), 4096 245 -> 200 (4), 16,384 202 ->
-// 178 (16); end positions of 8000 seeds in a 256^3 field 227 -> 191 (8), in F16 fields
-// that L2 holds 119 -> 121; pathlines of 8000 seeds 262 -> 214.
-inline uint32_t particles_per_warp(uint64_t count, int sms) {
-  uint32_t lanes = 1;
-  while (lanes < 32 && count > uint64_t(lanes) * 8u * uint64_t(sms)) lanes *= 2;
-  return lanes;
-}
-
 template <int kIntegrator, int kStorage, int kLocate, bool kRecord, bool kUnsteady, int kPPT>
 cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t stream) {
   // Persistent grid: as many blocks as fit on the device at once (or as the
@@ -396,7 +356,9 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
   const uint32_t own = free_shape ? particles_per_warp(a.count, sms) : 32u * kPPT;
   constexpr uint32_t threads = kLocate & kNarrowBit ? 64 : kAdvectBlock;
   const uint32_t block =
-      own < 32 ? 32 : advect_block(a, threads, lanes, sms, f.threads_per_sm ? 0 : resident);
+      own < 32 ? 32
+               : advect_block(a.block, a.blocks_per_sm, threads, lanes, sms,
+                              f.threads_per_sm ? 0 : resident);
   if (block == 0 || block % 32 != 0 || block > uint32_t(kAdvectBlock)) return cudaErrorInvalidValue;
   DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>(
       block, &resident, &sms)));

@@ -190,8 +190,8 @@ struct dpa_tuning_state {
   uint32_t blocks_per_sm = 0; // persistent grid: 0 = as many as fit
   uint32_t order = 64;        // processing order: Morton buckets of an order^3
                               // coarsening of the grid (1..64); 0: input order
-  uint32_t block = 0;         // threads per block (multiple of 32, <= 256); 0: 256, or
-                              // fewer so that a small launch reaches every SM
+  uint32_t block = 0;         // threads per block (multiple of 32, <= 256); 0: the
+                              // rules of launch_shape.hpp
   uint32_t particles_per_thread = 1;  // 1 or 2 (steady fields without recording)
 };
 

@@ -2,13 +2,10 @@
 #pragma once
 
 #include "common.cuh"
+#include "launch_shape.hpp"
 
 namespace dpa {
 
-#ifndef DPA_ADVECT_BLOCK
-#define DPA_ADVECT_BLOCK 256
-#endif
-constexpr int kAdvectBlock = DPA_ADVECT_BLOCK;
 #ifndef DPA_ADVECT_MIN_BLOCKS
 #define DPA_ADVECT_MIN_BLOCKS 4
 #endif
@@ -36,11 +33,6 @@ constexpr int kAdvectTrueRk4MinBlocks = DPA_ADVECT_TRUE_RK4_MIN_BLOCKS;
 #define DPA_ADVECT_PPT2_MIN_BLOCKS 2
 #endif
 constexpr int kAdvectPpt2MinBlocks = DPA_ADVECT_PPT2_MIN_BLOCKS;
-// Launches whose particles would fill fewer blocks than the device has SMs
-// use smaller blocks (1) or keep kAdvectBlock threads per block (0).
-#ifndef DPA_ADVECT_SPREAD
-#define DPA_ADVECT_SPREAD 1
-#endif
 
 struct AdvectArgs {
   uint64_t count;
@@ -55,8 +47,7 @@ struct AdvectArgs {
   uint32_t claim;                    // order entries a warp claims at once
   uint32_t blocks_per_sm;            // persistent grid per SM (0: occupancy maximum)
   uint32_t block;                    // threads per block: a multiple of 32 up to
-                                     // kAdvectBlock; 0 = kAdvectBlock, or fewer when
-                                     // the particles would not reach every SM
+                                     // kAdvectBlock; 0 = the rules of launch_shape.hpp
   uint32_t particles_per_thread;     // 1 or 2 (2: steady fields without recording)
   unsigned long long* work_counter;  // claims of the order; the launcher zeroes it, or
                                      // passes null when every particle has a slot

@@ -326,9 +326,12 @@ typedef struct dpa_tuning {
   uint32_t order;          /* processing order: Morton buckets of a order^3 coarsening
                               of the grid (1..64), 0 = input order */
   float    measured_ms;    /* dpa_autotune_advect: time of the chosen setting */
-  uint32_t block_size;     /* threads per block, a multiple of 32 up to 256; 0 = 256,
-                              or fewer when a launch's particles would not reach
-                              every SM */
+  uint32_t block_size;     /* threads per block, a multiple of 32 up to 256; 0 = by
+                              launch: 256, fewer when the particles would not reach
+                              every SM and, unless blocks_per_sm is given, 32 with
+                              fewer particles to a warp for the smallest launches
+                              and 64 where blocks of 256 would fit at once but
+                              unevenly and for pathlines that do not fit at once */
   uint32_t particles_per_thread; /* 1 or 2 particles stepped together by each lane
                               (2 applies to steady fields without recording) */
 } dpa_tuning;
