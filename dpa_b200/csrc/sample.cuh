@@ -615,6 +615,7 @@ template <int kIntegrator, class Sampler>
 __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& k,
                                    Sampler& sampler, Position& p, float t,
                                    StepHistory& history, bool active = true) {
+  constexpr bool kPacked = Sampler::kPackedSums;
   const float2 unit = make_float2(f.unit[0], f.unit[1]);
   float2 v01;
   float v2;
@@ -628,13 +629,19 @@ __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& 
     const bool zero = is_zero(v01, v2);
     Position n = p;
     if constexpr (kIntegrator == DPA_INTEGRATOR_EULER) {
+      // odeint euler: x = 1 * x + dt * dxdt
       n.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, v2));
-      n.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.dt), v01), unit);
+      n.p21 = advance<kPacked>(p.p21, mul2(splat(k.dt), v01), unit);
     } else {
+      // odeint runge_kutta4, final stage with four equal stage derivatives:
+      // x = 1 * x + (b0 dt) d + (b1 dt) d + (b2 dt) d + (b3 dt) d, left to right.
       const float m0 = __fmul_rn(k.c0, v2), m1 = __fmul_rn(k.c1, v2);
       n.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, m0), m1), m1), m0);
       const float2 n0 = mul2(splat(k.c0), v01), n1 = mul2(splat(k.c1), v01);
-      n.p21 = advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(p.p21, n0, unit), n1, unit), n1, unit), n0, unit);
+      n.p21 = advance<kPacked>(n.p21, n0, unit);
+      n.p21 = advance<kPacked>(n.p21, n1, unit);
+      n.p21 = advance<kPacked>(n.p21, n1, unit);
+      n.p21 = advance<kPacked>(n.p21, n0, unit);
     }
     const bool taken = active && inside && !zero;
     p.p0 = taken ? n.p0 : p.p0;
@@ -642,48 +649,39 @@ __device__ __forceinline__ int step(const FieldView& f, const StepCoefficients& 
     return !(active && inside) ? int(kStepOutOfBounds)
            : zero              ? int(kStepZeroVelocity)
                                : int(kStepTaken);
-  }
-  if (!sampler.sample(f, p, t, v01, v2)) return kStepOutOfBounds;
-  if (is_zero(v01, v2)) return kStepZeroVelocity;
-  if constexpr (kIntegrator == DPA_INTEGRATOR_EULER) {
-    // odeint euler: x = 1 * x + dt * dxdt
-    p.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, v2));
-    p.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.dt), v01), unit);
-  } else if constexpr (kIntegrator == DPA_INTEGRATOR_RUNGE_KUTTA_4) {
-    // odeint runge_kutta4, final stage with four equal stage derivatives:
-    // x = 1 * x + (b0 dt) d + (b1 dt) d + (b2 dt) d + (b3 dt) d, left to right.
-    const float m0 = __fmul_rn(k.c0, v2), m1 = __fmul_rn(k.c1, v2);
-    p.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, m0), m1), m1), m0);
-    const float2 n0 = mul2(splat(k.c0), v01), n1 = mul2(splat(k.c1), v01);
-    p.p21 = advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(p.p21, n0, unit), n1, unit), n1, unit), n0, unit);
-  } else if constexpr (kIntegrator == kGeneralIntegrator) {
-    general_step(k.g, v01, v2, history, p);
   } else {
-    // Four-sample RK4; a stage outside the grid ends the particle without
-    // taking the step.
-    float2 k2_01, k3_01, k4_01;
-    float k2_2, k3_2, k4_2;
-    Position x;
-    x.p0 = __fadd_rn(p.p0, __fmul_rn(k.half, v2));
-    x.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.half), v01), unit);
-    const float t_half = __fadd_rn(t, k.half), t_end = __fadd_rn(t, k.dt);
-    if (!sampler.sample(f, x, t_half, k2_01, k2_2)) return kStepOutOfBounds;
-    x.p0 = __fadd_rn(p.p0, __fmul_rn(k.half, k2_2));
-    x.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.half), k2_01), unit);
-    if (!sampler.sample(f, x, t_half, k3_01, k3_2)) return kStepOutOfBounds;
-    x.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, k3_2));
-    x.p21 = advance<Sampler::kPackedSums>(p.p21, mul2(splat(k.dt), k3_01), unit);
-    if (!sampler.sample(f, x, t_end, k4_01, k4_2)) return kStepOutOfBounds;
-    p.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, __fmul_rn(k.c0, v2)),
-                                         __fmul_rn(k.c1, k2_2)),
-                               __fmul_rn(k.c1, k3_2)),
-                     __fmul_rn(k.c0, k4_2));
-    const float2 C0 = splat(k.c0), C1 = splat(k.c1);
-    p.p21 = advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(advance<Sampler::kPackedSums>(p.p21, mul2(C0, v01), unit), mul2(C1, k2_01), unit),
-                      mul2(C1, k3_01), unit),
-                 mul2(C0, k4_01), unit);
+    if (!sampler.sample(f, p, t, v01, v2)) return kStepOutOfBounds;
+    if (is_zero(v01, v2)) return kStepZeroVelocity;
+    if constexpr (kIntegrator == kGeneralIntegrator) {
+      general_step(k.g, v01, v2, history, p);
+    } else {
+      // Four-sample RK4; a stage outside the grid ends the particle without
+      // taking the step.
+      float2 k2_01, k3_01, k4_01;
+      float k2_2, k3_2, k4_2;
+      Position x;
+      x.p0 = __fadd_rn(p.p0, __fmul_rn(k.half, v2));
+      x.p21 = advance<kPacked>(p.p21, mul2(splat(k.half), v01), unit);
+      const float t_half = __fadd_rn(t, k.half), t_end = __fadd_rn(t, k.dt);
+      if (!sampler.sample(f, x, t_half, k2_01, k2_2)) return kStepOutOfBounds;
+      x.p0 = __fadd_rn(p.p0, __fmul_rn(k.half, k2_2));
+      x.p21 = advance<kPacked>(p.p21, mul2(splat(k.half), k2_01), unit);
+      if (!sampler.sample(f, x, t_half, k3_01, k3_2)) return kStepOutOfBounds;
+      x.p0 = __fadd_rn(p.p0, __fmul_rn(k.dt, k3_2));
+      x.p21 = advance<kPacked>(p.p21, mul2(splat(k.dt), k3_01), unit);
+      if (!sampler.sample(f, x, t_end, k4_01, k4_2)) return kStepOutOfBounds;
+      p.p0 = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(p.p0, __fmul_rn(k.c0, v2)),
+                                           __fmul_rn(k.c1, k2_2)),
+                                 __fmul_rn(k.c1, k3_2)),
+                       __fmul_rn(k.c0, k4_2));
+      const float2 c0 = splat(k.c0), c1 = splat(k.c1);
+      p.p21 = advance<kPacked>(p.p21, mul2(c0, v01), unit);
+      p.p21 = advance<kPacked>(p.p21, mul2(c1, k2_01), unit);
+      p.p21 = advance<kPacked>(p.p21, mul2(c1, k3_01), unit);
+      p.p21 = advance<kPacked>(p.p21, mul2(c0, k4_01), unit);
+    }
+    return kStepTaken;
   }
-  return kStepTaken;
 }
 
 }  // namespace dpa
