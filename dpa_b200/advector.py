@@ -249,10 +249,12 @@ class _CurveCollector:
 
     def curve(self) -> IntegralCurve:
         itype = np.uint64 if self.index64 else np.uint32
-        vert = np.concatenate(self.vertices) if self.vertices else np.zeros((0, 3), np.float32)
-        col = np.concatenate(self.colors) if self.colors else np.zeros(0, np.float32)
-        idx = np.concatenate(self.indices) if self.indices else np.zeros(0, itype)
-        return IntegralCurve(vert, col, idx.astype(itype, copy=False))
+
+        def joined(parts, empty):
+            return parts[0] if len(parts) == 1 else np.concatenate(parts) if parts else empty
+        return IntegralCurve(joined(self.vertices, np.zeros((0, 3), np.float32)),
+                             joined(self.colors, np.zeros(0, np.float32)),
+                             joined(self.indices, np.zeros(0, itype)))
 
 
 LOAD_BALANCERS = ("none", "diffuse_constant", "diffuse_lesser_average",

@@ -336,38 +336,33 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
                 "set index64");
 
   // The piece's curve crosses to the host in chunks through two pinned halves, so
-  // that a chunk copies while the sink takes the one before it and the pinned memory
-  // stays bounded (dpa_context_set_host_chunk_limit). Chunks begin at 1 MiB of
-  // vertices and colors, which with its indices stays in a core's 2 MiB cache while
-  // the sink copies it on (260 MB in three rounds into the caller's arrays: 22.6 ms,
-  // against 24 to 25 at 2 MiB or in one chunk and 27.9 at 16 MiB), and double, to
-  // 16 MiB at most, whenever the next one had not landed when the sink returned: the
-  // copies then bound the round, and larger ones cost less (the same rounds,
-  // discarded: 6.4 ms in chunks of 1 MiB, 5.2 doubling).
+  // that chunk j + 1 copies while the sink takes chunk j and the pinned memory stays
+  // bounded (dpa_context_set_host_chunk_limit). Chunks are as large as the limit
+  // allows: a sink that appends them to vectors moves what it holds whenever the next
+  // one does not fit, so that 53 MB of curve take it 7 ms in one chunk and 55 in chunks
+  // of 1 MiB. A sink that copies into room of its own is faster with those (260 MB in
+  // three rounds 26 and 23 ms); its program sets the limit.
   if (sink) {
-    constexpr uint64_t kFirstChunk = 1ull << 20, kMostChunk = 16ull << 20;
-    const uint64_t most_v = std::max<uint64_t>(std::min(ctx->host_chunk_bytes, kMostChunk) / 16, 1);
-    const uint64_t most_i = std::max<uint64_t>(ctx->host_chunk_bytes / index_bytes, 2) & ~1ull;
-    uint64_t cap_v = std::min(most_v, kFirstChunk / 16);
-    auto cap_i = [&] { return std::min(most_i, 2 * cap_v); };
-    const uint64_t half_v = std::min(piece_vertices, most_v);
-    const uint64_t half_i = std::min({piece_indices, most_i, 2 * most_v});
+    const uint64_t cap_v = std::max<uint64_t>(ctx->host_chunk_bytes / 16, 1);
+    const uint64_t cap_i = std::max<uint64_t>(ctx->host_chunk_bytes / index_bytes, 2) & ~1ull;
+    const uint64_t chunks = std::max<uint64_t>(
+        {1, (piece_vertices + cap_v - 1) / cap_v, (piece_indices + cap_i - 1) / cap_i});
+    const uint64_t half_v = std::min(piece_vertices, cap_v);
+    const uint64_t half_i = std::min(piece_indices, cap_i);
     DPA_TRY_CUDA(ctx, ctx->host_vertices.reserve(2 * half_v * 12));
     DPA_TRY_CUDA(ctx, ctx->host_colors.reserve(2 * half_v * 4));
     DPA_TRY_CUDA(ctx, ctx->host_indices.reserve(2 * half_i * index_bytes));
     for (cudaEvent_t& ev : ctx->chunk_events)
       if (!ev) DPA_TRY_CUDA(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    struct {
+    auto span = [](uint64_t j, uint64_t cap, uint64_t total, uint64_t* first, uint64_t* count) {
+      *first = std::min(j * cap, total);
+      *count = std::min(cap, total - *first);
+    };
+    auto issue = [&](uint64_t j) -> int {
+      const uint64_t h = j & 1;
       uint64_t v0, vn, i0, in;
-    } span[2];
-    uint64_t next_v = 0, next_i = 0;
-    auto all_issued = [&] { return next_v == piece_vertices && next_i == piece_indices; };
-    auto issue = [&](uint64_t h) -> int {  // the next chunk, into half h
-      span[h] = {next_v, std::min(cap_v, piece_vertices - next_v), next_i,
-                 std::min(cap_i(), piece_indices - next_i)};
-      const auto [v0, vn, i0, in] = span[h];
-      next_v += vn;
-      next_i += in;
+      span(j, cap_v, piece_vertices, &v0, &vn);
+      span(j, cap_i, piece_indices, &i0, &in);
       if (vn) {
         DPA_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->host_vertices.as<float>() + 3 * h * half_v,
                                           ctx->out_vertices.as<float>() + 3 * v0, vn * 12,
@@ -387,29 +382,25 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
     };
     st = issue(0);
     if (st != DPA_OK) return st;
-    bool more = true;
-    for (uint64_t h = 0; more; h ^= 1) {
-      more = !all_issued();
-      if (more) {
-        st = issue(h ^ 1);  // into the half whose chunk the sink has returned
+    for (uint64_t j = 0; j < chunks; ++j) {
+      if (j + 1 < chunks) {
+        st = issue(j + 1);  // into the half whose chunk the sink has returned
         if (st != DPA_OK) return st;
       }
-      const cudaError_t landed = cudaEventQuery(ctx->chunk_events[h]);
-      if (landed == cudaErrorNotReady) {
-        if (span[h].v0) cap_v = std::min(2 * cap_v, most_v);
-        DPA_TRY_CUDA(ctx, cudaEventSynchronize(ctx->chunk_events[h]));
-      } else {
-        DPA_TRY_CUDA(ctx, landed);
-      }
+      const uint64_t h = j & 1;
+      DPA_TRY_CUDA(ctx, cudaEventSynchronize(ctx->chunk_events[h]));
+      uint64_t v0, vn, i0, in;
+      span(j, cap_v, piece_vertices, &v0, &vn);
+      span(j, cap_i, piece_indices, &i0, &in);
       dpa_curve_chunk c{};
-      c.vertex_offset = *round_vertices + span[h].v0;
-      c.vertex_count = span[h].vn;
+      c.vertex_offset = *round_vertices + v0;
+      c.vertex_count = vn;
       c.vertices = ctx->host_vertices.as<float>() + 3 * h * half_v;
       c.colors = o->colors ? ctx->host_colors.as<float>() + h * half_v : nullptr;
-      c.index_offset = *round_indices + span[h].i0;
-      c.index_count = span[h].in;
+      c.index_offset = *round_indices + i0;
+      c.index_count = in;
       c.indices = ctx->host_indices.as<char>() + h * half_i * index_bytes;
-      c.last = (final_piece && !more) ? 1 : 0;
+      c.last = (final_piece && j + 1 == chunks) ? 1 : 0;
       if (sink(user, &c) != 0) {
         cudaStreamSynchronize(s);  // no copy may still target the halves
         return fail(ctx, DPA_ERROR_SINK, "curve sink aborted the round");
