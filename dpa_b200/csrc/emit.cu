@@ -8,6 +8,8 @@
 // the reference's round curve: vertices in round-particle order, invalid
 // sentinels removed, index pairs (i, i + 1) for consecutive vertices neither
 // of which is the terminal sentinel, and one color per vertex.
+#include <cmath>
+
 #include "kernels.cuh"
 #include "sample.cuh"
 
@@ -317,7 +319,7 @@ __global__ void repack_kernel(const float* xyzv, uint64_t nodes, const FieldView
     const uint32_t i0 = row / uint32_t(f.n[1]), i1 = row - i0 * uint32_t(f.n[1]);
     at = copy = tiled_node(f.tile, i0, i1, i2);
     if (kStorage != DPA_STORAGE_F32_EDGES && i2 > 0 &&
-        __umulhi(i2, f.tile.magic[2]) != __umulhi(i2 - 1, f.tile.magic[2]))
+        tile_bits(f.tile, 2, float(i2)) != tile_bits(f.tile, 2, float(i2 - 1)))
       copy = uint64_t(tiled_node(f.tile, i0, i1, i2 - 1)) + 1;
   }
   auto store = [&](auto* o, auto v) {
@@ -432,7 +434,8 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& f,
 // 256 MB to 892 in one of 2 GB. Tiles keep a particle's path in fewer pages, and
 // fewer warps in flight leave room for their misses.
 uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
-  constexpr uint64_t kTileBytes = 512ull << 20, kFewerThreadsBytes = 1280ull << 20;
+  constexpr uint64_t kTileBytes = 512ull << 20;
+  constexpr uint64_t kFewerThreadsBytes = 1280ull << 20;
   const uint64_t node_bytes = field_node_bytes(v.storage);
   const uint64_t nodes = uint64_t(v.n[0]) * uint64_t(v.n[1]) * uint64_t(v.n[2]);
   v.tiled = 0;
@@ -455,16 +458,21 @@ uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
   const uint64_t tile = size[0] * size[1] * row;
   const uint64_t total = tile * tiles[0] * tiles[1] * tiles[2];
   v.threads_per_sm = 512;
-  // An axis of one node would need a magic of 2^32; the index is 32 bits wide.
+  // The index is 32 bits wide; an axis of one node has no cells.
   if (rows || size[0] < 2 || size[1] < 2 || size[2] < 2 || total >= (1ull << 32)) return nodes;
   v.threads_per_sm = total * node_bytes > kFewerThreadsBytes ? 768 : 0;
   v.tiled = 1;
-  for (int i = 0; i < 3; ++i) v.tile.magic[i] = uint32_t((1ull << 32) / size[i] + 1);
+  for (int i = 0; i < 3; ++i) {
+    v.tile.inverse[i] = 1.0f / float(size[i]);
+    if (double(v.tile.inverse[i]) * double(size[i]) < 1.0)
+      v.tile.inverse[i] = std::nextafter(v.tile.inverse[i], 2.0f);
+  }
   v.tile.stride[0] = uint32_t(size[1] * row);
   v.tile.stride[1] = uint32_t(row);
   v.tile.jump[0] = uint32_t(tiles[1] * tiles[2] * tile - size[0] * size[1] * row);
   v.tile.jump[1] = uint32_t(tiles[2] * tile - size[1] * row);
   v.tile.jump[2] = uint32_t(tile - size[2]);
+  v.tile.bias = 0u - 0x4B000000u * (v.tile.jump[0] + v.tile.jump[1] + v.tile.jump[2]);
   return total;
 }
 

@@ -83,9 +83,10 @@ __device__ __forceinline__ float remainder_general(float a, float s, float h) {
   return r;
 }
 
-// Subscripts of a cell's first node.
+// Subscripts of a cell's first node, and the same as floats.
 struct Cell {
   uint32_t i0, i1, i2;
+  float s[3];
 };
 
 // Where a position falls in the grid, per axis: the rounded quotient
@@ -125,7 +126,7 @@ __device__ __forceinline__ void floor_bits(const float q[3], float s[3], Cell& c
     s[k] = __fsub_rn(b, 0x1p23f);
     i[k] = __float_as_uint(b) - kTwo23;
   }
-  c = {i[0], i[1], i[2]};
+  c = {i[0], i[1], i[2], {s[0], s[1], s[2]}};
 }
 
 // Locates p; c receives its cell (meaningful only when p is inside).
@@ -179,11 +180,26 @@ __device__ __forceinline__ bool locate(const FieldView& f, const Position& p, Ce
   return (c.i0 < f.cells[0]) & (c.i1 < f.cells[1]) & (c.i2 < f.cells[2]);
 }
 
+// The tile of a subscript along an axis, plus the bits of 2^23 (TileLayout::bias takes
+// them off): s * inverse + 2^23 rounded down, as in floor_bits. inverse is 1 / size
+// rounded up, too large by less than 2^-23 / size, so that s * inverse never reaches the
+// next integer for s < 2^23.
+__device__ __forceinline__ uint32_t tile_bits(const TileLayout& t, int axis, float s) {
+  return __float_as_uint(__fmaf_rd(s, t.inverse[axis], 0x1p23f));
+}
+
 // Index, within its slice, of a node in tile order.
 __device__ __forceinline__ uint32_t tiled_node(const TileLayout& t, uint32_t i0, uint32_t i1,
                                                uint32_t i2) {
-  return i0 * t.stride[0] + __umulhi(i0, t.magic[0]) * t.jump[0] + i1 * t.stride[1] +
-         __umulhi(i1, t.magic[1]) * t.jump[1] + i2 + __umulhi(i2, t.magic[2]) * t.jump[2];
+  return i0 * t.stride[0] + tile_bits(t, 0, float(i0)) * t.jump[0] + i1 * t.stride[1] +
+         tile_bits(t, 1, float(i1)) * t.jump[1] + i2 + tile_bits(t, 2, float(i2)) * t.jump[2] +
+         t.bias;
+}
+
+// Index of a cell's first node in row order: what tells cells apart, in a tiled field
+// too, where the node's own index would cost three more products a sample.
+__device__ __forceinline__ uint32_t first_node(const FieldView& f, const Cell& c) {
+  return c.i0 * f.stride0 + c.i1 * f.stride1 + c.i2;
 }
 
 // Indices, within their slice, of the first nodes of a cell's four edges along
@@ -196,15 +212,15 @@ template <bool kTiled>
 __device__ __forceinline__ CellRows cell_rows(const FieldView& f, const Cell& c) {
   if constexpr (kTiled) {
     const TileLayout& t = f.tile;
-    auto along = [&](int axis, uint32_t i) {
-      return i * t.stride[axis] + __umulhi(i, t.magic[axis]) * t.jump[axis];
-    };
-    const uint32_t a0 = along(0, c.i0), a1 = along(0, c.i0 + 1);
-    const uint32_t z = c.i2 + __umulhi(c.i2, t.magic[2]) * t.jump[2];
-    const uint32_t b0 = along(1, c.i1) + z, b1 = along(1, c.i1 + 1) + z;
+    const uint32_t z = c.i2 + tile_bits(t, 2, c.s[2]) * t.jump[2] + t.bias;
+    const uint32_t r0 = c.i0 * t.stride[0] + z, r1 = c.i1 * t.stride[1];
+    const uint32_t a0 = r0 + tile_bits(t, 0, c.s[0]) * t.jump[0];
+    const uint32_t a1 = r0 + t.stride[0] + tile_bits(t, 0, c.s[0] + 1.0f) * t.jump[0];
+    const uint32_t b0 = r1 + tile_bits(t, 1, c.s[1]) * t.jump[1];
+    const uint32_t b1 = r1 + t.stride[1] + tile_bits(t, 1, c.s[1] + 1.0f) * t.jump[1];
     return {a0 + b0, a0 + b1, a1 + b0, a1 + b1};
   } else {
-    const uint32_t n = c.i0 * f.stride0 + c.i1 * f.stride1 + c.i2;
+    const uint32_t n = first_node(f, c);
     return {n, n + f.stride1, n + f.stride0, n + f.stride0 + f.stride1};
   }
 }
@@ -403,7 +419,7 @@ struct CellSampler {
   static constexpr int kLocate = kMode & ~kTiledBit;
   static constexpr bool kTiled = (kMode & kTiledBit) != 0;
   CornersOf<kStorage> corners;
-  uint32_t cached = ~0u;  // first node of the cached cell (no cell starts there)
+  uint32_t cached = ~0u;  // first_node of the cached cell (no cell starts there)
 
   // Samples at p (a steady field: the time t is not used); returns false
   // when p is outside the grid. The sample is returned as v01 = (v0, v1)
@@ -413,10 +429,10 @@ struct CellSampler {
     Cell c;
     Weights w;
     if (!locate<kLocate>(f, p, c, w)) return false;
-    const CellRows rows = cell_rows<kTiled>(f, c);
-    if (rows.at[0] != cached) {
-      gather<kStorage>(f, rows, corners);
-      cached = rows.at[0];
+    const uint32_t cell = first_node(f, c);
+    if (cell != cached) {
+      gather<kStorage>(f, cell_rows<kTiled>(f, c), corners);
+      cached = cell;
     }
     trilinear(f, corners, w, v01, v2);
     return true;
