@@ -429,13 +429,26 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& f,
 //   F32 768^3, 7.2 GB                           32.5 [1024], 16.8 [768], 17.0 [512]
 //   F16 512^3, 1.1 GB  15.9 [1024], 11.1 [768]  10.4 [1024], 11.3 [768]
 //   F16 768^3, 3.6 GB                           15.5 [1024], 13.6 [768]
-// Beyond about half a gigabyte the gathers of a full SM miss the address
+// and 500 steps of curl noise / of a field that varies over 8 nodes only:
+//   F32 330^3, 0.6 GB   6.6 / 5.8 [1024]        6.6 / 5.9 [1024]
+//   F16 420^3, 0.6 GB   6.0 / 5.5 [1024]        6.3 / 6.0 [1024]
+//   F16 512^3, 1.1 GB  12.0 / 5.6 [1024]        7.1 / 6.1 [1024],  7.7 / 6.3 [768]
+//   F16 640^3, 2.1 GB  18.0 / 5.8 [1024]        8.7 / 6.3 [1024],  9.1 / 6.6 [768]
+//   F16 768^3, 3.6 GB                          10.6 / 6.4 [1024],  9.9 / 6.9 [768]
+//   edges 260^3, 0.6 GB 5.1 / 4.5 [1024]        5.3 / 4.8 [1024],  5.8 / 5.0 [768]
+//   edges 400^3, 2.0 GB 16.7 / 4.7 [1024]       8.5 / 5.1 [1024],  8.6 / 5.5 [768]
+//   edges 450^3, 2.9 GB                         9.2 / 5.2 [1024],  9.0 / 5.6 [768]
+//   edges 500^3, 4.0 GB 19.4 / 5.2 [1024]      10.1 / 5.3 [1024],  9.5 / 5.8 [768]
+// (a lattice of 2 million seeds in edge records of 256^3, 0.5 GB: 2.6 in rows, 2.35 in
+// tiles). Beyond about half a gigabyte the gathers of a full SM miss the address
 // translation cache: random 16-byte gathers fall from 2079 GB/s in a table of
 // 256 MB to 892 in one of 2 GB. Tiles keep a particle's path in fewer pages, and
-// fewer warps in flight leave room for their misses.
+// fewer warps in flight leave room for their misses: above 1.25 GiB for F32 nodes, above
+// 3 GiB for the others, whose gathers are half as many or half as large and which have
+// more to lose where a field is smooth.
 uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
   constexpr uint64_t kTileBytes = 512ull << 20;
-  constexpr uint64_t kFewerThreadsBytes = 1280ull << 20;
+  const uint64_t fewer_threads_bytes = (v.storage == DPA_STORAGE_F32 ? 1280ull : 3072ull) << 20;
   const uint64_t node_bytes = field_node_bytes(v.storage);
   const uint64_t nodes = uint64_t(v.n[0]) * uint64_t(v.n[1]) * uint64_t(v.n[2]);
   v.tiled = 0;
@@ -460,7 +473,7 @@ uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
   v.threads_per_sm = 512;
   // The index is 32 bits wide; an axis of one node has no cells.
   if (rows || size[0] < 2 || size[1] < 2 || size[2] < 2 || total >= (1ull << 32)) return nodes;
-  v.threads_per_sm = total * node_bytes > kFewerThreadsBytes ? 768 : 0;
+  v.threads_per_sm = total * node_bytes > fewer_threads_bytes ? 768 : 0;
   v.tiled = 1;
   for (int i = 0; i < 3; ++i) {
     v.tile.inverse[i] = 1.0f / float(size[i]);
