@@ -313,7 +313,7 @@ int dpa_advect_batch_device(dpa_context* ctx, const dpa_field* field,
  * dpa_graph_launch replays it on a stream (NULL: the context's). The graph
  * owns its scratch (8 bytes per particle and about 1 MB), so the context's
  * other calls may run between replays; replays of one graph must not
- * overlap. dpa_graph_destroy waits for the device. */
+ * overlap. dpa_graph_destroy waits for the last replay, on whatever stream it is. */
 int dpa_graph_create_advect(dpa_context* ctx, const dpa_field* field,
                             const dpa_advect_options* options, uint64_t count,
                             float* device_positions, uint64_t* device_remaining,
