@@ -1505,8 +1505,9 @@ int dpa_graph_launch(dpa_context* ctx, dpa_graph* graph, void* stream) {
 int dpa_graph_destroy(dpa_context* ctx, dpa_graph* graph) {
   if (!ctx || !graph || graph->owner != ctx) return DPA_ERROR_INVALID_ARGUMENT;
   cudaSetDevice(ctx->device);
-  // Replays may run on any stream; the scratch goes only once they are done.
-  cudaDeviceSynchronize();
+  // Replays may run on any stream: cudaFree waits for them (a device-wide wait is
+  // forbidden while any thread captures a stream of the device).
+  graph->scratch.release();
   if (graph->exec) cudaGraphExecDestroy(graph->exec);
   if (graph->graph) cudaGraphDestroy(graph->graph);
   delete graph;
