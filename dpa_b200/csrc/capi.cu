@@ -341,7 +341,9 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
   // allows: a sink that appends them to vectors moves what it holds whenever the next
   // one does not fit, so that 53 MB of curve take it 7 ms in one chunk and 55 in chunks
   // of 1 MiB. A sink that copies into room of its own is faster with those (260 MB in
-  // three rounds 26 and 23 ms); its program sets the limit.
+  // three rounds 26 and 23 ms); its program sets the limit. A single chunk needs one half:
+  // pinning memory is most of a context's first round (its 13 MB of curve 25 ms with two
+  // halves, 12 with one; 100 MB 162 and 95).
   if (sink) {
     const uint64_t cap_v = std::max<uint64_t>(ctx->host_chunk_bytes / 16, 1);
     const uint64_t cap_i = std::max<uint64_t>(ctx->host_chunk_bytes / index_bytes, 2) & ~1ull;
@@ -349,9 +351,10 @@ int record_piece(dpa_context* ctx, const dpa_field* field, const dpa_advect_opti
         {1, (piece_vertices + cap_v - 1) / cap_v, (piece_indices + cap_i - 1) / cap_i});
     const uint64_t half_v = std::min(piece_vertices, cap_v);
     const uint64_t half_i = std::min(piece_indices, cap_i);
-    DPA_TRY_CUDA(ctx, ctx->host_vertices.reserve(2 * half_v * 12));
-    DPA_TRY_CUDA(ctx, ctx->host_colors.reserve(2 * half_v * 4));
-    DPA_TRY_CUDA(ctx, ctx->host_indices.reserve(2 * half_i * index_bytes));
+    const uint64_t halves = std::min<uint64_t>(chunks, 2);
+    DPA_TRY_CUDA(ctx, ctx->host_vertices.reserve(halves * half_v * 12));
+    DPA_TRY_CUDA(ctx, ctx->host_colors.reserve(halves * half_v * 4));
+    DPA_TRY_CUDA(ctx, ctx->host_indices.reserve(halves * half_i * index_bytes));
     for (cudaEvent_t& ev : ctx->chunk_events)
       if (!ev) DPA_TRY_CUDA(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     auto span = [](uint64_t j, uint64_t cap, uint64_t total, uint64_t* first, uint64_t* count) {

@@ -161,7 +161,7 @@ int dpa_context_set_staging_limit(dpa_context* ctx, uint64_t bytes);
 
 /* Upper bound on the curve bytes one sink chunk carries (default 256 MiB of
  * vertices and colors, and as many bytes of indices). A piece's curve crosses
- * to the host through two pinned buffers of this size, the next chunk copying
+ * to the host through up to two pinned buffers of this size, the next chunk copying
  * while the sink takes the current one. Chunks are as large as the limit allows;
  * a sink that copies them into room that it has already is faster with chunks of
  * 1 MiB, which overlap its copies and stay in a core's cache, while one that
