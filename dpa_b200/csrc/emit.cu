@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kScanThreads) offsets_tiles_kernel(
 }
 
 // The three passes as one block's, for few particles: launches cost more there
-// than the scan (4096 particles: three kernels and their gaps 9 us, this 5).
+// than the scan (kOneBlockOffsets).
 constexpr int kOneBlockThreads = 1024;
 __global__ void __launch_bounds__(kOneBlockThreads) offsets_one_block_kernel(
     const uint32_t* a, const uint32_t* b, uint64_t n, uint64_t* out_a, uint64_t* out_b,

@@ -150,6 +150,8 @@ struct EmitArgs {
   void* indices;                  // piece output (uint32 or uint64)
 };
 
+// (Discarded rounds with the scans and without, us: 60 particles 73 and 68, 1024 69.5
+// and 66.)
 constexpr uint64_t kEmitScans = 1024;
 cudaError_t launch_emit(const EmitArgs& e, bool index64, bool colors, cudaStream_t stream);
 
@@ -162,7 +164,9 @@ cudaError_t launch_curve_offsets(const uint32_t* kept_vertices, const uint32_t* 
                                  uint64_t count, void* scratch, uint64_t* vertex_offsets,
                                  uint64_t* segment_offsets, unsigned long long* totals,
                                  cudaStream_t stream);
-constexpr uint64_t kOneBlockOffsets = 8192;
+// One block or three launches, us a discarded round of 60 iterations: 2000 particles 154
+// and 158, 3000 184 and 186, 3600 206 and 203, 4096 224 and 217, 8192 371 and 354.
+constexpr uint64_t kOneBlockOffsets = 3072;
 inline int curve_offsets_launches(uint64_t count) { return count <= kOneBlockOffsets ? 1 : 3; }
 
 // The data-path probe of dpa_measure_gather_bandwidth: blocks x 256 lanes,
