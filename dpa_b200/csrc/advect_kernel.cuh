@@ -392,8 +392,11 @@ cudaError_t launch_ppt(const FieldView& f, const AdvectArgs& a, cudaStream_t s) 
   if constexpr (advect_has_narrow<kIntegrator, kStorage, kRecord, kUnsteady>()) {
     // Narrow where the wide kernel cannot hold every particle at once; where it can,
     // a launch lasts as long as its longest chain of steps, and the spills lengthen
-    // that (8000 pathlines 600 -> 608 us). A tuning's launch shape is the wide
-    // kernel's. A launch of nothing prepares both.
+    // that (8000 pathlines 600 -> 608 us; of 300 steps, wide and narrow: 60,000 292 and
+    // 294, edge records 75,776 295 and 303). Beyond it 76,000 take 409 and 340 us, edge
+    // records 411 and 342, 100,000 505 and 486, 470 and 459, 300,000 1135 and 1058, 1020
+    // and 907. A tuning's launch shape is the wide kernel's. A launch of nothing prepares
+    // both.
     int sms = 0, resident = 0;
     DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, 1>(
         kAdvectBlock, &resident, &sms)));

@@ -148,11 +148,16 @@ constexpr uint64_t kEarlyEmitBytes = 4ull << 20;
 
 // Rounds of up to this many particles pass through pinned memory, one copy each
 // way; the driver stages each of the arrays of a larger one itself, or takes them
-// from pinned memory of the caller's.
+// from pinned memory of the caller's, which would lose by a copy from here on. End
+// positions of 20 steps, us without and with staging, from ordinary arrays: 2000 seeds 91
+// and 56, 16,384 203 and 132, 30,000 313 and 215, 131,072 988 and 850; from pinned ones: 74
+// and 54, 108 and 109, 129 and 156, 356 and 660.
 constexpr uint64_t kStagedParticles = 16384;
 
 // A staged round whose curve would take no more than this if every particle lived
-// to its last iteration comes back whole, with the end states.
+// to its last iteration comes back whole, with the end states: one wait instead of two
+// or three (discarded rounds, us: 60 seeds of 100 iterations 96 -> 68, 3000 of 20 129 ->
+// 99). What particles that leave early do not fill crosses the link too, 38 us at most.
 constexpr uint64_t kWholeCurveBytes = 2ull << 20;
 
 // Raw (unpruned) vertex offsets of n particles, remaining + 2 slots each, and
