@@ -17,13 +17,15 @@ same metric through the host C ABI call (dpa_advect_round) with pinned host
 buffers, copies included. The CPU baseline is the oracle's reference-faithful
 restatement on a bounded seed sample on the host cores.
 
-The same line carries the other configurations, each with its own device
-rate, end-to-end rate, CPU baseline timed in this run and error against the
-FP64 oracle: `recording` (64^3 ABC, 4096 seeds x 1000 steps, curves with
-uint32 indices), `ftle` (256^3 ABC + noise, 128^3 lattice x 250 steps, FTLE),
-`batched` (512^3 curl noise, 64 seed sets, 16 M particles, recording with
-uint64 indices, graph-captured autotuned launches) and `serving` (resident
-fields, Poisson arrivals, p50/p99 latency over three seeded runs).
+The other configurations follow, each with its own device rate, end-to-end
+rate, CPU baseline timed in this run and error against the FP64 oracle:
+`recording` (64^3 ABC, 4096 seeds x 1000 steps, curves with uint32 indices),
+`ftle` (256^3 ABC + noise, 128^3 lattice x 250 steps, FTLE), `batched` (512^3
+curl noise, 64 seed sets, 16 M particles, recording with uint64 indices,
+graph-captured autotuned launches) and `serving` (resident fields, Poisson
+arrivals, p50/p99 latency over three seeded runs). The line on standard output
+holds their main figures (`configurations`) and stays short, so that a log's
+tail holds it whole; the full report goes to standard error as one JSON object.
 `--workload NAME` prints one of them alone.
 """
 from __future__ import annotations
@@ -1193,6 +1195,38 @@ def _cuda_available():
         return False
 
 
+REPORT_ONLY = ("precision_forms", "fp64_error", "true_rk4", "systems_forms", "recording", "ftle",
+               "batched", "serving")
+
+
+def headline(report):
+    """The line of standard output: the report without its long parts, whose main figures
+    stand under `configurations`."""
+    line = {k: v for k, v in report.items() if k not in REPORT_ONLY}
+    main = {}
+    for name in ("recording", "ftle", "batched"):
+        if name in report:
+            r = report[name]
+            main[name] = {"value": r["value"], "unit": r["unit"], "ms_per_step": r["ms_per_step"],
+                          "e2e": r["e2e"]["value"], "cpu_baseline": r["cpu_baseline"]["value"]}
+    if "batched" in main:
+        main["batched"]["f16"] = report["batched"]["f16"]["particle_steps_per_s"]
+        main["batched"]["plain_f32"] = report["batched"]["plain_f32"]["particle_steps_per_s"]
+    if "serving" in report:
+        r = report["serving"]
+        main["serving"] = {"latency_ms": {k: r["latency_ms"][k] for k in ("p50_pooled",
+                                                                          "p99_pooled")},
+                           "particle_steps_per_s": r["particle_steps_per_s"]}
+    if "precision_forms" in report:
+        main["kernel_ms"] = {k: v["kernel_ms"] for k, v in report["precision_forms"].items()
+                             if "kernel_ms" in v}
+    if "true_rk4" in report:
+        main["true_rk4"] = report["true_rk4"]["particle_steps_per_s"]
+    if main:
+        line["configurations"] = main
+    return line
+
+
 def run_one(a):
     """One configuration alone (--workload recording / ftle / batched / serving)."""
     import torch
@@ -1366,7 +1400,8 @@ def run_gpu(a):
             out["batched"] = batched_config(ctx, stream, a)
             out["serving"] = serving_config(a, ctx)
     if rank == 0:
-        print(json.dumps(out), flush=True)
+        print(json.dumps(out), file=sys.stderr, flush=True)
+        print(json.dumps(headline(out)), flush=True)
     if field is not None:
         field.close()
     ctx.close()
