@@ -419,7 +419,9 @@ struct CellSampler {
   static constexpr int kLocate = kMode & ~kTiledBit;
   static constexpr bool kTiled = (kMode & kTiledBit) != 0;
   CornersOf<kStorage> corners;
-  uint32_t cached = ~0u;  // first_node of the cached cell (no cell starts there)
+  // What tells the cached cell: its first_node, or where its first node lies
+  // (sample_selected, which forms that in any case). No cell starts at ~0.
+  uint32_t cached = ~0u;
 
   // Samples at p (a steady field: the time t is not used); returns false
   // when p is outside the grid. The sample is returned as v01 = (v0, v1)
