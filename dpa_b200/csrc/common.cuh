@@ -73,8 +73,9 @@ struct FieldView {
   uint32_t cells[3];       // n - 1, the cells per axis
   int32_t tiled;           // the nodes are in `tile` order
   TileLayout tile;
+  alignas(8) float unit[2]; // {1, 1}: a multiplier the compiler cannot see (sample.cuh); a
+                            // pair, which the packed FMAs read as one 64-bit operand
   uint32_t threads_per_sm; // the most a launch keeps resident by default (0: no limit)
-  float unit[2];           // {1, 1}: a multiplier the compiler cannot see (sample.cuh)
   int32_t storage;         // dpa_storage
   // LocateMode of the spatial axes. kLocatePow2 needs every spacing a power
   // of two in [2^-20, 2^20] and every offset zero or at least 2^-100 in
