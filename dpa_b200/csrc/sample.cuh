@@ -196,8 +196,8 @@ __device__ __forceinline__ uint32_t tiled_node(const TileLayout& t, uint32_t i0,
          t.bias;
 }
 
-// Index of a cell's first node in row order: what tells cells apart, in a tiled field
-// too, where the node's own index would cost three more products a sample.
+// Index of a cell's first node in row order: tells cells apart also in a tiled field, where
+// the node's own index would cost three more products a sample.
 __device__ __forceinline__ uint32_t first_node(const FieldView& f, const Cell& c) {
   return c.i0 * f.stride0 + c.i1 * f.stride1 + c.i2;
 }
@@ -419,8 +419,8 @@ struct CellSampler {
   static constexpr int kLocate = kMode & ~kTiledBit;
   static constexpr bool kTiled = (kMode & kTiledBit) != 0;
   CornersOf<kStorage> corners;
-  // What tells the cached cell: its first_node, or where its first node lies
-  // (sample_selected, which forms that in any case). No cell starts at ~0.
+  // What tells the cached cell: where its first node lies, or its first_node in sample()
+  // of a tiled field. No cell starts at ~0.
   uint32_t cached = ~0u;
 
   // Samples at p (a steady field: the time t is not used); returns false
@@ -431,10 +431,18 @@ struct CellSampler {
     Cell c;
     Weights w;
     if (!locate<kLocate>(f, p, c, w)) return false;
-    const uint32_t cell = first_node(f, c);
-    if (cell != cached) {
-      gather<kStorage>(f, cell_rows<kTiled>(f, c), corners);
-      cached = cell;
+    if constexpr (kTiled) {
+      const uint32_t cell = first_node(f, c);
+      if (cell != cached) {
+        gather<kStorage>(f, cell_rows<true>(f, c), corners);
+        cached = cell;
+      }
+    } else {
+      const CellRows rows = cell_rows<false>(f, c);
+      if (rows.at[0] != cached) {
+        gather<kStorage>(f, rows, corners);
+        cached = rows.at[0];
+      }
     }
     trilinear(f, corners, w, v01, v2);
     return true;
