@@ -353,19 +353,19 @@ cudaError_t launch_typed(const FieldView& f, const AdvectArgs& a, cudaStream_t s
   DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>(
       kAdvectBlock, &resident, &sms)));
   const bool free_shape = kPPT == 1 && !a.block && !a.blocks_per_sm;
+  const uint32_t limit = limited_threads(f.threads_per_sm, f.limit_speed, a.coefficients.dt);
   const uint32_t own = free_shape ? particles_per_warp(a.count, sms) : 32u * kPPT;
   constexpr uint32_t threads = kLocate & kNarrowBit ? 64 : kAdvectBlock;
   const uint32_t block =
       own < 32 ? 32
                : advect_block(a.block, a.blocks_per_sm, threads, lanes, sms,
-                              f.threads_per_sm ? 0 : resident);
+                              limit ? 0 : resident);
   if (block == 0 || block % 32 != 0 || block > uint32_t(kAdvectBlock)) return cudaErrorInvalidValue;
   DPA_CUDA_TRY((resident_blocks<kIntegrator, kStorage, kLocate, kRecord, kUnsteady, kPPT>(
       block, &resident, &sms)));
   if (a.count == 0) return cudaSuccess;  // nothing to do, or preparation only
   if (a.blocks_per_sm && int(a.blocks_per_sm) < resident) resident = int(a.blocks_per_sm);
-  if (!a.blocks_per_sm && f.threads_per_sm)
-    resident = std::min(resident, std::max(1, int(f.threads_per_sm / block)));
+  if (!a.blocks_per_sm && limit) resident = std::min(resident, std::max(1, int(limit / block)));
   const uint64_t per_block = uint64_t(block / 32) * own;
   const uint64_t needed = (a.count + per_block - 1) / per_block;
   const uint64_t blocks = std::min<uint64_t>(needed, uint64_t(resident) * uint64_t(sms));

@@ -421,6 +421,44 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& f,
   }
 }
 
+namespace {
+
+constexpr int kSpeedBlocks = 64, kSpeedThreads = 256, kSpeedNodes = 4;  // per thread
+
+// The sampled nodes are the golden-ratio sequence over the field: evenly spread and in no
+// step with its rows.
+__global__ void __launch_bounds__(kSpeedThreads) field_speed_kernel(
+    const float* xyzv, uint64_t nodes, float s0, float s1, float s2, double* sums) {
+  const float per_cell[3] = {1.0f / s2, 1.0f / s1, 1.0f / s0};  // components in reversed order
+  double sum = 0.0;
+  for (int j = 0; j < kSpeedNodes; ++j) {
+    const uint64_t i = (uint64_t(blockIdx.x) * kSpeedThreads + threadIdx.x) * kSpeedNodes + j;
+    const float* at = xyzv + 3 * __umul64hi(i * 0x9E3779B97F4A7C15ull, nodes);
+    for (int c = 0; c < 3; ++c) {
+      const double v = double(at[c]) * double(per_cell[c]);
+      if (isfinite(v)) sum += v * v;
+    }
+  }
+  __shared__ double warps[kSpeedThreads / 32];
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31u) == 0) warps[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  sum = 0.0;
+  for (double w : warps) sum += w;
+  atomicAdd(sums, sum);
+  atomicAdd(sums + 1, double(kSpeedThreads * kSpeedNodes));
+}
+
+}  // namespace
+
+cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, const float spacing[3],
+                               double* sums, cudaStream_t stream) {
+  field_speed_kernel<<<kSpeedBlocks, kSpeedThreads, 0, stream>>>(xyzv, nodes, spacing[0], spacing[1],
+                                                                 spacing[2], sums);
+  return cudaGetLastError();
+}
+
 // Where the lines lie, measured on curl noise with 2 million seeds of up to 1000
 // steps of a quarter cell (rows, tiles; threads per SM in brackets, ms):
 //   F32 320^3, 0.5 GB   9.0 [1024]             9.0 [1024]
@@ -444,16 +482,21 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& f,
 // translation cache: random 16-byte gathers fall from 2079 GB/s in a table of
 // 256 MB to 892 in one of 2 GB. Tiles keep a particle's path in fewer pages, and
 // fewer warps in flight leave room for their misses: above 1.25 GiB for F32 nodes, above
-// 3 GiB for the others, whose gathers are half as many or half as large and which have
-// more to lose where a field is smooth.
+// 3 GiB for the others, whose gathers are half as many or half as large. Between those
+// the others gain by it where a step is long, and lose where particles stay in a cell
+// (limited_threads, launch_shape.hpp): 300 steps of 2 million seeds, ms in rows and at
+// 1024 and 768 threads, of curl noise at 0.6 cells a step, F16 580^3 20.7, 13.3, 9.0, edges
+// 400^3 19.8, 13.2, 8.5; of noise over 8 nodes at 0.25, 4.7, 4.5, 5.0 and 4.5, 4.1, 4.6. F32
+// nodes at 450^3, 1.5 GB: 24.8, 16.8, 11.9 and 6.2, 4.2, 4.6.
 uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
   constexpr uint64_t kTileBytes = 512ull << 20;
-  const uint64_t fewer_threads_bytes = (v.storage == DPA_STORAGE_F32 ? 1280ull : 3072ull) << 20;
+  constexpr uint64_t kFewerThreadsBytes = 1280ull << 20, kAlwaysFewerBytes = 3072ull << 20;
   const uint64_t node_bytes = field_node_bytes(v.storage);
   const uint64_t nodes = uint64_t(v.n[0]) * uint64_t(v.n[1]) * uint64_t(v.n[2]);
   v.tiled = 0;
   v.tile = TileLayout{};
   v.threads_per_sm = 0;
+  v.limit_speed = 0.0f;
   if (slices != 1 || nodes * node_bytes < kTileBytes) return nodes * slices;
   // About 64 nodes an axis, of a 2 MiB page for F32 nodes (axis 2: 32); tiles of
   // one axis are as even as they can be, and a row of one tile ends in no node of the
@@ -473,7 +516,10 @@ uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
   v.threads_per_sm = 512;
   // The index is 32 bits wide; an axis of one node has no cells.
   if (rows || size[0] < 2 || size[1] < 2 || size[2] < 2 || total >= (1ull << 32)) return nodes;
-  v.threads_per_sm = total * node_bytes > fewer_threads_bytes ? 768 : 0;
+  const uint64_t bytes = total * node_bytes;
+  v.threads_per_sm = bytes > kFewerThreadsBytes ? 768 : 0;
+  if (v.threads_per_sm && v.storage != DPA_STORAGE_F32 && bytes <= kAlwaysFewerBytes)
+    v.limit_speed = 1.0f;
   v.tiled = 1;
   for (int i = 0; i < 3; ++i) {
     v.tile.inverse[i] = 1.0f / float(size[i]);

@@ -188,9 +188,15 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& vi
                           cudaStream_t stream);
 
 // The layout of a steady field of this shape and storage, or of its rows. Returns the
-// nodes to allocate; sets view.tiled, view.tile and view.threads_per_sm (view.n and
-// view.storage are set).
+// nodes to allocate; sets view.tiled, view.tile, view.threads_per_sm and, to 1 where it is yet
+// to be measured, view.limit_speed (view.n and view.storage are set).
 uint64_t choose_layout(FieldView& view, uint32_t slices, bool rows);
+
+// Adds up, over a sample of the nodes of an XYZV field, the squared speeds in cells per
+// time (sums[0], components that are not finite left out) and the nodes (sums[1]). sums:
+// two zeroed doubles on the device.
+cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, const float spacing[3],
+                               double* sums, cudaStream_t stream);
 
 struct FtleArgs {
   uint64_t count;

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #ifndef DPA_ADVECT_BLOCK
@@ -48,6 +49,20 @@ inline uint32_t advect_block(uint32_t tuned_block, uint32_t tuned_blocks_per_sm,
   (void)resident;
 #endif
   return block;
+}
+
+// Threads per SM that a launch of steps of dt keeps resident (0: as many as fit), by the
+// field's limit and, where that depends on the steps, its RMS speed in cells per time. A
+// third of a cell a step is where nodes of 16 bits and edge records between 1.25 and 3
+// GiB begin to gain by fewer threads. 200 steps of 2 million seeds, us at 1024 and 768:
+//   F16 580^3, curl noise      0.3 cells 3899 and 4089, 0.35 4341 and 4250, 0.5 6451 and 4889
+//   F16 700^3                  0.3 4755 and 4576, 0.35 5671 and 4824
+//   edges 350^3                0.3 3467 and 3712, 0.35 3713 and 3876, 0.4 4040 and 4042
+//   edges 450^3                0.3 4587 and 4413, 0.35 5160 and 4666, 0.5 7418 and 5714
+//   F16 580^3, noise over 8 nodes only
+//                              0.3 3390 and 3729, 0.35 3537 and 3792, 0.5 4007 and 3961
+inline uint32_t limited_threads(uint32_t limit, float speed, float dt) {
+  return speed == 0.0f || std::fabs(dt) * speed > 1.0f / 3.0f ? limit : 0;
 }
 
 // Particles per warp of a small launch: as few as keep every SM at 8 warps or
