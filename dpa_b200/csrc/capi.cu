@@ -678,17 +678,18 @@ static int reciprocal_divides_exactly(dpa_context* ctx, float h, bool* exact) {
   return DPA_OK;
 }
 
-// RMS speed of a field's nodes in cells per time, never 0.
-static cudaError_t measure_speed(const float* xyzv, uint64_t nodes, const float spacing[3],
-                                 cudaStream_t s, float* speed) {
+// The speed that a field's limit of threads goes by, never 0.
+static cudaError_t measure_speed(const float* xyzv, uint64_t nodes, uint32_t n2,
+                                 const float spacing[3], cudaStream_t s, float* speed) {
   DeviceBuffer sums;
-  double total[2] = {0.0, 0.0};
+  double total[3] = {0.0, 0.0, 0.0};
   DPA_CUDA_TRY(sums.reserve(sizeof total));
   DPA_CUDA_TRY(cudaMemsetAsync(sums.ptr, 0, sizeof total, s));
-  DPA_CUDA_TRY(dpa::launch_field_speed(xyzv, nodes, spacing, sums.as<double>(), s));
+  DPA_CUDA_TRY(dpa::launch_field_speed(xyzv, nodes, n2, spacing, sums.as<double>(), s));
   DPA_CUDA_TRY(cudaMemcpyAsync(total, sums.ptr, sizeof total, cudaMemcpyDeviceToHost, s));
   DPA_CUDA_TRY(cudaStreamSynchronize(s));
-  *speed = float(std::clamp(std::sqrt(total[0] / total[1]), 1e-30, 1e30));
+  const double v = dpa::limit_speed(std::sqrt(total[0] / total[2]), std::sqrt(total[1] / total[2]));
+  *speed = float(std::clamp(v, 1e-30, 1e30));
   return cudaSuccess;
 }
 
@@ -746,7 +747,8 @@ static int create_field(dpa_context* ctx, const float* xyzv, bool device_input,
     if (e == cudaSuccess)
       e = dpa::launch_repack(src, nodes, f->view, f->nodes.ptr, ctx->stream);
     if (e == cudaSuccess && f->view.limit_speed != 0.0f)
-      e = measure_speed(src, nodes, spacing, ctx->stream, &f->view.limit_speed);
+      e = measure_speed(src, nodes, uint32_t(shape[2]), spacing, ctx->stream,
+                        &f->view.limit_speed);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     // A program that makes fields over and over again needs the copy's block again too.
     if (e == cudaSuccess && (kept || copy_kept)) staging.release_to(ctx->spare);

@@ -92,8 +92,8 @@ struct FieldView {
   int32_t time_fast;         // the time axis divides as kLocateReciprocal
   float time_upper;          // slices - 1: inside iff 0 <= (t - t0) / dt < slices - 1
   uint32_t time_cells;       // the same as an integer
-  float limit_speed;         // where threads_per_sm depends on a launch's steps: the RMS speed
-                             // in cells per time (limited_threads, launch_shape.hpp); else 0
+  float limit_speed;         // where threads_per_sm depends on a launch's steps: the speed
+                             // in cells per time that it goes by (launch_shape.hpp); else 0
 };
 
 // a / h by a known divisor: with y + yl = 1 / h split into two floats,

@@ -428,34 +428,41 @@ constexpr int kSpeedBlocks = 64, kSpeedThreads = 256, kSpeedNodes = 4;  // per t
 // The sampled nodes are the golden-ratio sequence over the field: evenly spread and in no
 // step with its rows.
 __global__ void __launch_bounds__(kSpeedThreads) field_speed_kernel(
-    const float* xyzv, uint64_t nodes, float s0, float s1, float s2, double* sums) {
+    const float* xyzv, uint64_t nodes, uint32_t n2, float s0, float s1, float s2, double* sums) {
   const float per_cell[3] = {1.0f / s2, 1.0f / s1, 1.0f / s0};  // components in reversed order
-  double sum = 0.0;
+  double sum[2] = {0.0, 0.0};
   for (int j = 0; j < kSpeedNodes; ++j) {
     const uint64_t i = (uint64_t(blockIdx.x) * kSpeedThreads + threadIdx.x) * kSpeedNodes + j;
-    const float* at = xyzv + 3 * __umul64hi(i * 0x9E3779B97F4A7C15ull, nodes);
+    uint64_t node = __umul64hi(i * 0x9E3779B97F4A7C15ull, nodes);
+    if (node % n2 + 1 == n2) --node;  // a row's last node has none behind it
+    const float* at = xyzv + 3 * node;
     for (int c = 0; c < 3; ++c) {
       const double v = double(at[c]) * double(per_cell[c]);
-      if (isfinite(v)) sum += v * v;
+      const double next = double(at[3 + c]) * double(per_cell[c]);
+      if (!isfinite(v) || !isfinite(next)) continue;
+      sum[0] += v * v;
+      sum[1] += (next - v) * (next - v);
     }
   }
-  __shared__ double warps[kSpeedThreads / 32];
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31u) == 0) warps[threadIdx.x >> 5] = sum;
+  __shared__ double warps[2][kSpeedThreads / 32];
+  for (int k = 0; k < 2; ++k) {
+    for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    if ((threadIdx.x & 31u) == 0) warps[k][threadIdx.x >> 5] = sum[k];
+  }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  sum = 0.0;
-  for (double w : warps) sum += w;
-  atomicAdd(sums, sum);
-  atomicAdd(sums + 1, double(kSpeedThreads * kSpeedNodes));
+  if (threadIdx.x >= 2) return;
+  double total = 0.0;
+  for (double w : warps[threadIdx.x]) total += w;
+  atomicAdd(sums + threadIdx.x, total);
+  if (threadIdx.x == 0) atomicAdd(sums + 2, double(kSpeedThreads * kSpeedNodes));
 }
 
 }  // namespace
 
-cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, const float spacing[3],
-                               double* sums, cudaStream_t stream) {
-  field_speed_kernel<<<kSpeedBlocks, kSpeedThreads, 0, stream>>>(xyzv, nodes, spacing[0], spacing[1],
-                                                                 spacing[2], sums);
+cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, uint32_t n2,
+                               const float spacing[3], double* sums, cudaStream_t stream) {
+  field_speed_kernel<<<kSpeedBlocks, kSpeedThreads, 0, stream>>>(
+      xyzv, nodes, n2, spacing[0], spacing[1], spacing[2], sums);
   return cudaGetLastError();
 }
 
@@ -484,7 +491,7 @@ cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, const float sp
 // fewer warps in flight leave room for their misses: above 1.25 GiB for F32 nodes, above
 // 3 GiB for the others, whose gathers are half as many or half as large. Between those
 // the others gain by it where a step is long, and lose where particles stay in a cell
-// (limited_threads, launch_shape.hpp): 300 steps of 2 million seeds, ms in rows and at
+// (launch_shape.hpp): 300 steps of 2 million seeds, ms in rows and at
 // 1024 and 768 threads, of curl noise at 0.6 cells a step, F16 580^3 20.7, 13.3, 9.0, edges
 // 400^3 19.8, 13.2, 8.5; of noise over 8 nodes at 0.25, 4.7, 4.5, 5.0 and 4.5, 4.1, 4.6. F32
 // nodes at 450^3, 1.5 GB: 24.8, 16.8, 11.9 and 6.2, 4.2, 4.6.

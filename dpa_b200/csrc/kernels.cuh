@@ -193,10 +193,11 @@ cudaError_t launch_repack(const float* xyzv, uint64_t nodes, const FieldView& vi
 uint64_t choose_layout(FieldView& view, uint32_t slices, bool rows);
 
 // Adds up, over a sample of the nodes of an XYZV field, the squared speeds in cells per
-// time (sums[0], components that are not finite left out) and the nodes (sums[1]). sums:
-// two zeroed doubles on the device.
-cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, const float spacing[3],
-                               double* sums, cudaStream_t stream);
+// time (sums[0]) and their squared changes to the next node along axis 2, of n2 >= 2
+// nodes (sums[1]), components that are not finite left out, and the nodes (sums[2]). sums:
+// three zeroed doubles on the device.
+cudaError_t launch_field_speed(const float* xyzv, uint64_t nodes, uint32_t n2,
+                               const float spacing[3], double* sums, cudaStream_t stream);
 
 struct FtleArgs {
   uint64_t count;

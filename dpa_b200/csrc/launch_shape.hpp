@@ -52,9 +52,10 @@ inline uint32_t advect_block(uint32_t tuned_block, uint32_t tuned_blocks_per_sm,
 }
 
 // Threads per SM that a launch of steps of dt keeps resident (0: as many as fit), by the
-// field's limit and, where that depends on the steps, its RMS speed in cells per time. A
-// third of a cell a step is where nodes of 16 bits and edge records between 1.25 and 3
-// GiB begin to gain by fewer threads. 200 steps of 2 million seeds, us at 1024 and 768:
+// field's limit and, where that depends on the steps, a speed in cells per time. A third
+// of a cell a step is where nodes of 16 bits and edge records between 1.25 and 3 GiB begin
+// to gain by fewer threads while neighbouring particles stay together. 200 steps of 2
+// million seeds, us at 1024 and 768 threads:
 //   F16 580^3, curl noise      0.3 cells 3899 and 4089, 0.35 4341 and 4250, 0.5 6451 and 4889
 //   F16 700^3                  0.3 4755 and 4576, 0.35 5671 and 4824
 //   edges 350^3                0.3 3467 and 3712, 0.35 3713 and 3876, 0.4 4040 and 4042
@@ -63,6 +64,19 @@ inline uint32_t advect_block(uint32_t tuned_block, uint32_t tuned_blocks_per_sm,
 //                              0.3 3390 and 3729, 0.35 3537 and 3792, 0.5 4007 and 3961
 inline uint32_t limited_threads(uint32_t limit, float speed, float dt) {
   return speed == 0.0f || std::fabs(dt) * speed > 1.0f / 3.0f ? limit : 0;
+}
+
+// That speed, of a field's RMS speed and the RMS change of its velocity from a node to the
+// next. Where the velocity changes by more than a twentieth in a cell, particles part on
+// their way and gather from everywhere: the line lies at a fifth of a cell a step. Curl
+// noise, 400 and 2000 steps of 2 million seeds, ms at 1024 and 768 threads:
+//   F16 580^3    0.16 cells 5.8 and 6.6, 24.2 and 27.5; 0.22 6.3 and 6.9, 28.9 and 28.3
+//   F16 700^3    0.16 6.4 and 7.1, 26.8 and 29.6; 0.22 7.1 and 7.6, 40.0 and 31.2
+//   edges 450^3  0.16 6.0 and 6.6, 24.5 and 26.0; 0.22 6.9 and 7.1, 31.3 and 27.9
+// and at 0.3 cells, 2000 steps, 52 and 33, 67 and 42, 61 and 33; noise over 8 nodes only, 0.25
+// cells, 2000 steps, 19.4 and 21.2, 20.5 and 22.9, 15.8 and 17.7.
+inline double limit_speed(double speed, double change) {
+  return change > 0.05 * speed ? speed * (5.0 / 3.0) : speed;
 }
 
 // Particles per warp of a small launch: as few as keep every SM at 8 warps or

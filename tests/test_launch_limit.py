@@ -12,9 +12,12 @@ DRIVER = r"""
 #include <cstdio>
 #include <cstdlib>
 #include "launch_shape.hpp"
-int main(int, char** argv) {
-  std::printf("%u", dpa::limited_threads(uint32_t(atoi(argv[1])), strtof(argv[2], 0),
-                                         strtof(argv[3], 0)));
+int main(int argc, char** argv) {
+  if (argc == 3)
+    std::printf("%.17g", dpa::limit_speed(strtod(argv[1], 0), strtod(argv[2], 0)));
+  else
+    std::printf("%u", dpa::limited_threads(uint32_t(atoi(argv[1])), strtof(argv[2], 0),
+                                           strtof(argv[3], 0)));
 }
 """
 
@@ -37,3 +40,21 @@ def test_limit(driver, limit, speed, dt, threads):
     out = subprocess.run([driver, str(limit), str(speed), str(dt)], capture_output=True, text=True,
                          check=True).stdout
     assert int(out) == threads
+
+
+# A field whose velocity changes by more than a twentieth in a cell is limited from a fifth
+# of a cell a step on.
+@pytest.mark.parametrize("speed,change,cells", [
+    (1.0, 0.0, 1 / 3), (1.0, 0.049, 1 / 3), (1.0, 0.051, 0.2), (3.0, 0.14, 1 / 3), (3.0, 2.0, 0.2),
+    (0.0, 0.0, None)])
+def test_speed(driver, speed, change, cells):
+    out = float(subprocess.run([driver, str(speed), str(change)], capture_output=True, text=True,
+                               check=True).stdout)
+    if cells is None:
+        assert out == 0.0
+        return
+    for factor, threads in ((0.999, 0), (1.001, 768)):
+        dt = factor * cells / speed
+        got = subprocess.run([driver, "768", str(out), str(dt)], capture_output=True, text=True,
+                             check=True).stdout
+        assert int(got) == threads
