@@ -44,12 +44,14 @@ constexpr int kNarrowBit = 8;
 // rows, so that the particles of an SM stay in few pages. Node (i0, i1, i2) of a
 // slice is at
 //   sum over axes of i * stride + (i / size) * jump   (stride 1 along axis 2),
-// the quotient i / size being the floor of i * inverse (tile_bits, sample.cuh).
+// the quotient i / size being the floor of i * inverse (tile_bits, sample.cuh), or the high
+// word of i * magic (i < 2^23, size <= 64).
 // Where axis 2 has several tiles, a tile's rows of nodes hold one node more than the
 // tile, the next tile's first, so that a cell's two nodes along it always follow each
 // other.
 struct TileLayout {
   float inverse[3];
+  uint32_t magic[3];
   uint32_t stride[2];
   uint32_t jump[3];
   uint32_t bias;  // takes the bits of 2^23 off the three quotients

@@ -532,6 +532,7 @@ uint64_t choose_layout(FieldView& v, uint32_t slices, bool rows) {
     v.tile.inverse[i] = 1.0f / float(size[i]);
     if (double(v.tile.inverse[i]) * double(size[i]) < 1.0)
       v.tile.inverse[i] = std::nextafter(v.tile.inverse[i], 2.0f);
+    v.tile.magic[i] = uint32_t((1ull << 32) / size[i] + 1);
   }
   v.tile.stride[0] = uint32_t(size[1] * row);
   v.tile.stride[1] = uint32_t(row);
